@@ -115,6 +115,12 @@ struct Geo {
     static constexpr int SLOT = NB * LD;  // elements per smem matrix slot
 };
 
+}  // namespace bss
+
+#include "bss_chol_f64.cuh"
+
+namespace bss {
+
 __device__ __forceinline__ void fma_vec(float &acc, const float4 &x, const float4 &y)
 {
     acc = fmaf(x.x, y.x, acc);
@@ -306,9 +312,8 @@ __device__ __forceinline__ T safe_pivot(T p)
 // ---------------------------------------------------------------------------
 
 // 1/sqrt of a pivot: the hardware approximation in FP32 (2 ulp; FP32
-// factors are refined in FP64 or checked at 1e-4), IEEE sqrt and divide in FP64
+// factors are refined in FP64 or checked at 1e-4)
 __device__ __forceinline__ float rsqrt_pivot(float p) { return rsqrtf(p); }
-__device__ __forceinline__ double rsqrt_pivot(double p) { return 1.0 / sqrt(p); }
 
 // 16-wide panels measured faster than 32-wide ones on GB300 for NB = 64
 // (24k vs 30k cycles per 64x64 factorization in one CTA): the warp
@@ -441,51 +446,6 @@ template <class T, int LD, int NB, int PB>
 __device__ __noinline__ void trailing_update(T *sS, int o, int tid, int nthr)
 {
     trailing_update_i<T, LD, NB, PB>(sS, o, tid, nthr);
-}
-
-// off-diagonal tiles of V = U^{-1} after the factorization (FP64 chains):
-// V_IJ = -V_II sum_{P=I+1..J} U_IP V_PJ, one super-diagonal stage at a time
-// (s = J - I), all threads on every stage; T_IJ is kept in the (scratch)
-// lower tile (J, I) of sS.  On GB300's FP64 pipe a warp-instruction costs
-// its full slot whatever lanes are active, so FP64 takes this form, whose
-// element-parallel stages skip the zero halves of the triangular tiles.
-template <class T, int LD, int NB, int PB>
-__device__ __noinline__ void inverse_stages(T *sS, T *sV, int tid, int nthr)
-{
-    constexpr int KP = NB / PB;
-#pragma unroll 1
-    for (int s = 1; s < KP; ++s) {
-        const int ntile = KP - s;
-        for (int e = tid; e < ntile * PB * PB; e += nthr) {
-            const int tile = e / (PB * PB), w = e - tile * PB * PB;
-            const int a = w % PB, b = w / PB;
-            const int I = tile, J = tile + s;
-            T acc0 = T(0), acc1 = T(0);
-            for (int P = I + 1; P <= J; ++P)
-#pragma unroll
-                for (int q = 0; q < PB; q += 2) {
-                    acc0 = fma(sS[(PB * I + a) + (PB * P + q) * LD], sV[(PB * P + q) + (PB * J + b) * LD], acc0);
-                    acc1 = fma(sS[(PB * I + a) + (PB * P + q + 1) * LD], sV[(PB * P + q + 1) + (PB * J + b) * LD],
-                               acc1);
-                }
-            sS[(PB * J + a) + (PB * I + b) * LD] = acc0 + acc1;
-        }
-        __syncthreads();
-        for (int e = tid; e < ntile * PB * PB; e += nthr) {
-            const int tile = e / (PB * PB), w = e - tile * PB * PB;
-            const int a = w % PB, b = w / PB;
-            const int I = tile, J = tile + s;
-            T acc0 = T(0), acc1 = T(0);
-            for (int c = a; c < PB; c += 2) {
-                acc0 = fma(sV[(PB * I + a) + (PB * I + c) * LD], sS[(PB * J + c) + (PB * I + b) * LD], acc0);
-                if (c + 1 < PB)
-                    acc1 = fma(sV[(PB * I + a) + (PB * I + c + 1) * LD], sS[(PB * J + c + 1) + (PB * I + b) * LD],
-                               acc1);
-            }
-            sV[(PB * I + a) + (PB * J + b) * LD] = -(acc0 + acc1);
-        }
-        __syncthreads();
-    }
 }
 
 // Off-diagonal block column J of V = U^{-1} (rows I < J), from V U = I:
@@ -706,7 +666,7 @@ __device__ __forceinline__ void inv_column_par(float *sS, float *sV, int J, int 
 // factors the diagonal tile while (FP32) the other warps form V's block
 // column K-1; then warp 1 inverts the diagonal tile while the rest solve the
 // row panel; then the trailing update.  V's last block column follows the
-// loop (FP32); FP64 forms V's off-diagonal tiles in stages after it.
+// loop.  FP64 tiles take f64_chol_inv (bss_chol_f64.cuh) instead.
 // The FAST form of tiles of 128 and more looks one panel ahead: once panel
 // K's row panel is solved, warp 0 updates only the next diagonal tile and
 // factors it at once, while the other warps update the rest of the trailing
@@ -721,8 +681,8 @@ __device__ __forceinline__ void inv_column_par(float *sS, float *sV, int J, int 
 // above; the named barrier 1 joins the THREADS - 32 threads that form V's
 // block columns during the panels.
 // `idle(K)` runs on warps 1.. while warp 0 factors diagonal tile K and they
-// have nothing else to do (panel-by-panel order: K < 2 in FP32, every K in
-// FP64): the caller's own work, which must not touch sS, sV or dinv.
+// have nothing else to do (panel-by-panel order: K < 2): the caller's own
+// work, which must not touch sS, sV or dinv.
 struct CholNoIdle {
     __device__ __forceinline__ void operator()(int) const {}
 };
@@ -733,6 +693,9 @@ __device__ __forceinline__ int chol_inv_blocked(T *sS, T *sV, T *dinv, int *sfla
 {
     static_assert(!FAST || (INL && sizeof(T) == 4), "the fast forms are inlined FP32");
     static_assert(THREADS > 32, "two warps at least");
+    if constexpr (sizeof(T) == 8) {
+        return f64_chol_inv<NB, THREADS>(sS, sV, sflag, tid);
+    } else {
     constexpr int LD = Geo<T, NB>::LD;
     constexpr int PB = Panel<NB>::PB;
     constexpr int KP = NB / PB;
@@ -782,7 +745,7 @@ __device__ __forceinline__ int chol_inv_blocked(T *sS, T *sV, T *dinv, int *sfla
             else
                 bad = warp_chol<T, LD, PB>(sS, dinv, o, lane);
             if (bad && lane == 0) *sflag = 1;
-        } else if (K >= 2 && sizeof(T) == 4) {
+        } else if (K >= 2) {
             if constexpr (FAST)
                 inv_column_par<LD, PB>(sS, sV, K - 1, tid - 32, THREADS - 32, 1);
             else if constexpr (INL)
@@ -817,9 +780,7 @@ __device__ __forceinline__ int chol_inv_blocked(T *sS, T *sV, T *dinv, int *sfla
         }
         __syncthreads();
     }
-    if constexpr (sizeof(T) == 8) {
-        inverse_stages<T, LD, NB, PB>(sS, sV, tid, THREADS);
-    } else if (KP > 1) {
+    if (KP > 1) {
         if constexpr (FAST)
             inv_column_par<LD, PB>(sS, sV, KP - 1, tid, THREADS, 0);
         else if constexpr (INL)
@@ -829,6 +790,7 @@ __device__ __forceinline__ int chol_inv_blocked(T *sS, T *sV, T *dinv, int *sfla
         __syncthreads();
     }
     return *sflag;
+    }
     }
 }
 

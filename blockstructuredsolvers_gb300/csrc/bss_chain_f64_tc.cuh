@@ -1,0 +1,570 @@
+// Chain factor kernel for FP64 factors of 17..64-wide blocks with the chain
+// step's products on the 5th-generation tensor cores: the same recursion and
+// outputs as chain_factor_body (V_i, W_i, Y_i, S_LL / S_RR / S_LR; also the
+// sequential coarsest chain), one CTA per partition.
+//
+// What bounds it: GB300's FP64 pipe retires 1.7 FMA per clock and SM, so the
+// five n^3 products of a 64-wide step took ~460K of its ~560K cycles.  FP16
+// MMAs run 2400 times faster, and an FP64 product can be put together from
+// FP16 products exactly (error-free splitting: Ozaki, Ogita, Oishi, Rump,
+// Numer. Algorithms 59, 2012): every operand row is scaled by a power of two
+// to |x| < 1 and cut into seven 8-bit digits,
+//     x = sum_{s=0..6} d_s 2^-(6 + 8 s),   d_s an integer, |d_0| <= 64, |d_s| <= 128,
+// which are exact in FP16; the products of digits s and t with s + t = l
+// form level l, whose 64-term sums are integers below 2^23 and so exact in
+// the FP32 accumulator of the MMA.  Levels 0..7 (34 digit products; level 8 is
+// 2^-59 of the largest term) are put together in 64-bit integers and rounded
+// to FP64 once.  Error: the digits hold 54 bits below the power of two above
+// the row's largest element (a whole FP64 mantissa there), so a product of
+// random rows is off by ~2^-54 of the largest terms, against ~2^-53 for the
+// 64 roundings of an FP64 FMA chain.  Rows with an infinity or NaN give NaN.
+//
+// A step of the chain (NB = 64 or 32, the block padded with the identity):
+//   P1 = [W_{i-1} | Y_{i-1}]^T W_{i-1}   -> S = A_i - W^T W (slot 0 rows), Z_i^T = -Y^T W (slot 1 rows)
+//   PL = [W_{i-1} | Y_{i-1}]^T Y_{i-1}   -> S_LL += Y^T Y (slot 1 rows), during the first pivot tile
+//   Cholesky + inverse V_i on the FP64 pipe (f64_chol_inv), Z_i and B_i cut into digits beside it
+//   P2 = [Z_i | B_i]^T V_i               -> Y_i^T (slot 0 rows), W_i^T (slot 1 rows)
+//
+// Operand layout (FP16, K-major, no swizzle, core matrices of 8 rows x 16
+// bytes, those of an 8-row group adjacent along K): digit s of slot j's row
+// group g is at ((s NB/8 + g) 2 + j) GRP with GRP = 16 NB bytes.  As the A
+// operand the groups of both slots follow one another (stride GRP: 128 MMA
+// rows, slots alternating every 8); as the B operand one slot's groups of
+// all digits do (stride 2 GRP), so one MMA with N = 64 J multiplies a digit of
+// A with J digits of B and its J results land in J consecutive levels'
+// accumulator columns.  The 34 digit products of a K-step are 12 MMAs instead
+// of 34 and 64-column MMAs at a third of the rate are avoided.
+//
+// TMEM: 8 levels x NB columns (all 512 for NB = 64).  Shared memory: 214 KB
+// (NB = 64, one CTA per SM), 58 KB (NB = 32; 128 registers allow two CTAs).
+//
+// Measured (the digit products of one operand pair: 4.7K cycles for NB = 64,
+// 1.4K for NB = 32, against 131K and 16K for one product on the FP64 pipe):
+// plain FP64 factor + solve of N = 16384, n = 64: 35.6 -> 13.3 ms; N = 1531,
+// n = 37, k = 3: 6.42 -> 2.77 ms; N = 100, n = 32: 679 -> 476 us.
+#pragma once
+
+namespace bss {
+
+constexpr int SL_DIGITS = 7, SL_LEVELS = 8, SL_THREADS = 256;
+constexpr int SL_NAN = 1 << 20;  // row exponent of a row with an infinity or a NaN
+
+template <int NB>
+struct SlGeo {
+    static constexpr int LD = Geo<double, NB>::LD;
+    static constexpr uint32_t GRP = 16u * NB;                    // 8 rows x NB digits
+    static constexpr uint32_t SLICE = 2u * (NB / 8) * GRP;       // one digit of both slots
+    static constexpr uint32_t VSLICE = (NB / 8) * GRP;           // one digit of the V operand
+    static constexpr uint32_t TILE = (uint32_t)Geo<double, NB>::SLOT * 8u;  // sS, X, sV
+    static constexpr uint32_t OFF_S = SL_DIGITS * SLICE;         // sS; after the Cholesky sS and X hold the V operand
+    static constexpr uint32_t OFF_X = OFF_S + TILE;              // Z in FP64; after P2 (sS, sX) hold W and Y in FP64
+    static constexpr uint32_t OFF_V = OFF_X + TILE;              // sV
+    static constexpr uint32_t OFF_EX = OFF_V + TILE;             // row exponents: slot 0, slot 1, V
+    static constexpr uint32_t OFF_CTL = OFF_EX + 3u * 64u * 4u;
+    static constexpr uint32_t BYTES = OFF_CTL + 64u;
+    static constexpr uint32_t TMEM = SL_LEVELS * NB;
+    static_assert(SL_DIGITS * VSLICE <= 2 * TILE, "the V operand overlays sS and X");
+};
+
+__device__ __forceinline__ uint64_t sl_desc(uint32_t saddr, uint32_t sbo)
+{
+    uint64_t d = (uint64_t)((saddr & 0x3FFFFu) >> 4);
+    d |= (uint64_t)(128u >> 4) << 16;  // leading byte offset: next core matrix along K
+    d |= (uint64_t)(sbo >> 4) << 32;   // stride byte offset: next 8-row group
+    d |= (uint64_t)1 << 46;            // descriptor version of the sm_100 family
+    return d;
+}
+
+// kind::f16, D = F32, A = B = F16, both K-major, M = 128
+__host__ __device__ constexpr uint32_t sl_idesc(int N)
+{
+    return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((128u >> 4) << 24);
+}
+
+__device__ __forceinline__ void sl_mma1(uint32_t tm, uint64_t da, uint64_t db, uint32_t idesc, uint32_t acc)
+{
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tm),
+        "l"(da), "l"(db), "r"(idesc), "r"(acc)
+        : "memory");
+}
+
+// every digit product of levels 0..7: A = both slots' rows at a, B = the NB
+// rows per digit at b with 8-row groups bsbo bytes apart; one thread
+template <int NB>
+__device__ __forceinline__ void sl_mma(uint32_t tm, uint32_t a, uint32_t b, uint32_t bsbo)
+{
+    using G = SlGeo<NB>;
+    constexpr int JMAX = 256 / NB;  // digits of B per MMA
+    const uint32_t bslice = (NB / 8) * bsbo;
+#pragma unroll 1
+    for (int kk = 0; kk < NB / 16; ++kk) {
+#pragma unroll
+        for (int s = 0; s < SL_DIGITS; ++s) {
+            const uint64_t da = sl_desc(a + s * G::SLICE + kk * 256u, G::GRP);
+            const int J = SL_LEVELS - s < SL_DIGITS ? SL_LEVELS - s : SL_DIGITS;
+            // digit 0 of A opens levels 0..6, digit 1 opens level 7 (with digit 6 of B)
+            const int split = s == 1 ? J - 1 : J;
+#pragma unroll
+            for (int j = 0; j < J;) {
+                const int end = j < split ? split : J;
+                const int cnt = end - j < JMAX ? end - j : JMAX;
+                const bool opens = s == 0 || (s == 1 && j == split);
+                sl_mma1(tm + (uint32_t)((s + j) * NB), da, sl_desc(b + j * bslice + kk * 256u, bsbo),
+                        sl_idesc(cnt * NB), (opens && kk == 0) ? 0u : 1u);
+                j += cnt;
+            }
+        }
+    }
+}
+
+// value v 2^e as FP64 (one rounding, to nearest); NaN for the marked exponents
+__device__ __forceinline__ double sl_to_f64(long long v, int e)
+{
+    const unsigned long long u0 = (unsigned long long)(v < 0 ? -v : v);
+    const unsigned uh = (unsigned)(u0 >> 32), ul = (unsigned)u0;
+    const int lz = uh ? __clz((int)uh) : 32 + __clz((int)ul);
+    const unsigned long long u = u0 << (lz & 63);
+    const unsigned long long q = (u >> 11) + ((u >> 10) & 1ull);  // 53 bits, the top one set
+    const int be = e + 63 - lz + 1023;
+    unsigned long long bits = ((unsigned long long)(unsigned)(be - 1) << 52) + q;
+    if (be <= 0) {  // subnormal
+        const int s = 12 - be;
+        bits = s > 63 ? 0ull : (u >> s) + ((u >> (s - 1)) & 1ull);
+    }
+    if (be >= 2047) bits = 0x7FF0000000000000ull;
+    if (u0 == 0) bits = 0;
+    if (v < 0) bits |= 0x8000000000000000ull;
+    if (e >= SL_NAN / 2) bits = 0x7FF8000000000000ull;
+    return __longlong_as_double((long long)bits);
+}
+
+// eight accumulator columns of this thread's TMEM lane, all levels -> FP64:
+// row exponent er, column exponents ec[0..7]
+template <int NB>
+__device__ __forceinline__ void sl_read8(uint32_t addr, int er, const int *ec, double (&out)[8])
+{
+    uint32_t r[SL_LEVELS][8];
+#pragma unroll
+    for (int l = 0; l < SL_LEVELS; ++l)
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=r"(r[l][0]), "=r"(r[l][1]), "=r"(r[l][2]), "=r"(r[l][3]), "=r"(r[l][4]), "=r"(r[l][5]),
+                       "=r"(r[l][6]), "=r"(r[l][7])
+                     : "r"(addr + (uint32_t)(l * NB)));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    // FP32 integers to int32 through the bits of f + 1.5 2^23 (|f| <= 2^22: levels
+    // 0..4, by 64 (|d_0| 128 2 + 128 128 (pairs - 2))); levels 5..7 reach 6 2^20:
+    // 5 in two parts, 6 and 7 halved (their last bit is 2^-60 and less).  The
+    // conversion instruction takes ~30 cycles of a scheduler, an add one.
+    constexpr float C23 = 12582912.f, C24 = 25165824.f;
+    constexpr unsigned B23 = 0x4B400000u, B24 = 0x4BC00000u;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        unsigned b[SL_LEVELS];
+#pragma unroll
+        for (int l = 0; l < 5; ++l) b[l] = __float_as_uint(__uint_as_float(r[l][q]) + C23);
+        {
+            const float f = __uint_as_float(r[5][q]), f2 = f + C24;  // f2: f to even
+            const float rest = f - (f2 - C24);
+            b[5] = 2u * __float_as_uint(f2) + __float_as_uint(rest + C23);
+        }
+#pragma unroll
+        for (int l = 6; l < 8; ++l) b[l] = __float_as_uint(fmaf(__uint_as_float(r[l][q]), 0.5f, C23));
+        // two levels each, |t| < 2^31
+        const int t0 = (int)(b[0] * 256u + b[1] - (B23 * 256u + B23));
+        const int t1 = (int)(b[2] * 256u + b[3] - (B23 * 256u + B23));
+        const int t2 = (int)(b[4] * 256u + b[5] - (B23 * 256u + 2u * B24 + B23));
+        const int t3 = (int)(b[6] * 256u + b[7] - (B23 * 256u + B23));  // halved
+        // unit 2^-56 (level l has unit 2^-(12 + 8 l)); |v| <= 2^62
+        const long long v = (long long)((unsigned long long)(long long)t0 << 36) + (long long)t1 * (1 << 20) + (long long)t2 * 16 + (t3 >> 11);
+        out[q] = sl_to_f64(v, er + ec[q] - 56);
+    }
+}
+
+// the largest exponent field (at least 1) of a row as stored: the power of
+// two above the row's largest element
+__device__ __forceinline__ int sl_row_exp(int emax) { return emax == 2047 ? SL_NAN : emax - 1022; }
+
+// eight consecutive K values of one operand row as digits: 16 bytes per
+// digit at dst + s * stride.  emax: the row's largest exponent field.
+__device__ __forceinline__ void sl_put8(unsigned char *dst, uint32_t stride, const double (&x)[8], int emax)
+{
+    uint32_t lo[8], hi[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const unsigned xh = (unsigned)__double2hiint(x[q]), xl = (unsigned)__double2loint(x[q]);
+        const int E = (int)((xh >> 20) & 0x7FFu);
+        const unsigned mh = (xh & 0xFFFFFu) | (E ? 0x100000u : 0u);
+        int sh = emax - (E ? E : 1);
+        sh = sh > 63 ? 63 : sh;
+        unsigned long long m = (((unsigned long long)mh << 32) | xl) << 2;
+        m = ((m >> sh) + 1) >> 1;  // |x| 2^54 / 2^(row exponent), rounded
+        const unsigned long long b = ((xh >> 31) ? 0ull - m : m) + 0x0080808080808080ull;  // byte 6 - s = digit s + 128
+        lo[q] = (uint32_t)b;
+        hi[q] = (uint32_t)(b >> 32);
+    }
+#pragma unroll
+    for (int s = 0; s < SL_DIGITS; ++s) {
+        const int byte = 6 - s;
+        uint32_t w[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const uint32_t a = byte < 4 ? lo[2 * u] : hi[2 * u], c = byte < 4 ? lo[2 * u + 1] : hi[2 * u + 1];
+            const unsigned k = (unsigned)(byte & 3);
+            // two FP16 numbers 1024 + byte, less 1024 + 128
+            const uint32_t p = (__byte_perm(a, c, k | ((4u + k) << 8)) & 0x00FF00FFu) | 0x64006400u;
+            asm("add.f16x2 %0, %1, %2;" : "=r"(w[u]) : "r"(p), "r"(0xE480E480u));
+        }
+        *reinterpret_cast<uint4 *>(dst + s * stride) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+}
+
+// one warp cuts eight operand rows into digits (lane: row lane % 8, quarter
+// lane / 8 of K) at dst (the row group's first core matrix of digit 0), their
+// exponents to exps[0..7].  row: the lane's row, its K values kstride apart,
+// zero from kvalid on.  Out of line: five callers, and the step's code should
+// stay in the instruction cache.
+template <int NB>
+__device__ __noinline__ void sl_cut_group(unsigned char *dst, uint32_t stride, int *exps, const double *row,
+                                          long long kstride, int kvalid)
+{
+    constexpr int KE = NB / 4;
+    const int lane = threadIdx.x & 31, k0 = (lane >> 3) * KE;
+    double x[KE];
+    int emax = 1 << 20;
+#pragma unroll
+    for (int q = 0; q < KE; ++q) {
+        x[q] = k0 + q < kvalid ? row[(k0 + q) * kstride] : 0.0;
+        emax = max(emax, __double2hiint(x[q]) & 0x7FFFFFFF);
+    }
+    emax = max(emax, __shfl_xor_sync(0xFFFFFFFFu, emax, 8));
+    emax = max(emax, __shfl_xor_sync(0xFFFFFFFFu, emax, 16));
+    emax >>= 20;
+    if (lane < 8) exps[lane] = sl_row_exp(emax);
+#pragma unroll
+    for (int q = 0; q < KE; q += 8) {
+        const double x8[8] = {x[q], x[q + 1], x[q + 2], x[q + 3], x[q + 4], x[q + 5], x[q + 6], x[q + 7]};
+        sl_put8(dst + (uint32_t)((k0 + q) / 8) * 128u + (uint32_t)(lane & 7) * 16u, stride, x8, emax);
+    }
+    fence_async_smem();
+}
+
+struct SlCtx {
+    uint32_t tm;      // TMEM base
+    C64Bar bM, bL;    // P1 / P2 (thread 0 waits), PL (thread 128 waits)
+    int *abort;
+};
+
+// one partition's chain (or the whole sequential chain when g.seq)
+template <int NB>
+__device__ __forceinline__ void chain_f64_tc_body(const ChainFactorArgs<double, double> &g, const long long p, SlCtx &cx)
+{
+    using G = SlGeo<NB>;
+    constexpr int LD = G::LD, HC = NB / 2, NW = SL_THREADS / 32;
+    extern __shared__ __align__(128) unsigned char smem_sl[];
+    unsigned char *OP = smem_sl;                                   // the operand slots
+    double *sS = reinterpret_cast<double *>(smem_sl + G::OFF_S);
+    double *sX = reinterpret_cast<double *>(smem_sl + G::OFF_X);
+    double *sV = reinterpret_cast<double *>(smem_sl + G::OFF_V);
+    unsigned char *OV = smem_sl + G::OFF_S;                        // the V operand
+    int *ex0 = reinterpret_cast<int *>(smem_sl + G::OFF_EX), *ex1 = ex0 + 64, *exV = ex1 + 64;
+    int *sflag = reinterpret_cast<int *>(smem_sl + G::OFF_CTL);
+    const uint32_t aOP = smem_u32(OP), aOV = smem_u32(OV);
+
+    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+    const int L = 32 * (w & 3) + lane;               // accumulator row
+    const bool live = L < 2 * NB;                    // (warp-uniform: NB = 32 uses rows 0-63)
+    const int slot = (L >> 3) & 1, m = (L >> 4) * 8 + (L & 7);  // its operand slot and row there
+    const int c0 = HC * (w >> 2);                    // its first accumulator column
+    const uint32_t tl = cx.tm + ((uint32_t)(32 * (w & 3)) << 16);
+    const int n = g.n;
+    const long long nn = (long long)n * n;
+    const bool seq = g.seq != 0;
+    long long first, last, sL = 0;
+    if (seq) {
+        first = 0;
+        last = g.N - 1;
+    } else {
+        sL = (p * (g.N - 1)) / g.Q;
+        const long long sR = ((p + 1) * (g.N - 1)) / g.Q;
+        first = sL + 1;
+        last = sR - 1;
+    }
+    double *Cp = seq ? nullptr : g.C + p * 3 * nn;
+    for (int e = tid; e < Geo<double, NB>::SLOT; e += SL_THREADS) sV[e] = 0.0;  // V's strictly lower tiles stay zero
+    __syncthreads();
+
+    // S_LL (+)= Y^T Y from the PL accumulator, by warps 4-7 (named barrier 3)
+    auto add_sll = [&](bool add) {
+        if (tid == 128) c64_wait1(cx.bL, cx.abort);
+        asm volatile("bar.sync 3, 128;" ::: "memory");
+        if (*cx.abort || !live) return;
+        tc_fence_after();
+        const int er = ex1[m];
+#pragma unroll 1
+        for (int q0 = 0; q0 < NB; q0 += 8) {
+            double v[8];
+            sl_read8<NB>(tl + (uint32_t)q0, er, ex1 + q0, v);
+            if (slot == 1 && m < n) {
+#pragma unroll
+                for (int q = 0; q < 8; ++q)
+                    if (q0 + q < n) {
+                        double *c = Cp + m + (long long)(q0 + q) * n;
+                        *c = add ? *c + v[q] : v[q];
+                    }
+            }
+        }
+        tc_fence_before();
+    };
+    auto issue_pl = [&]() {
+        if (tid == 128) {  // (not warp 0: an MMA holds its issuing thread for its duration)
+            tc_fence_after();
+            sl_mma<NB>(cx.tm, aOP, aOP + G::GRP, 2 * G::GRP);
+            tc_commit(cx.bL.addr);
+            cx.bL.pending = true;
+        }
+    };
+
+    // A_i into sS (identity outside n x n), asynchronously, by warps 1-7
+    auto fetch_a = [&](long long i) {
+        const double *Ag = g.A_in + i * nn;
+        if (w == 0) return;
+        if (n == NB && ((uintptr_t)Ag & 15u) == 0) {
+            for (int e = tid - 32; e < NB * NB / 2; e += SL_THREADS - 32)
+                cp_async16(sS + 2 * (e % (NB / 2)) + (e / (NB / 2)) * LD, Ag + 2 * e);
+        } else {
+            for (int e = tid - 32; e < NB * NB; e += SL_THREADS - 32) {
+                const int r = e % NB, c = e / NB;
+                if (r < n && c < n)
+                    cp_async8(sS + r + c * LD, Ag + r + (long long)c * n);
+                else
+                    sS[r + c * LD] = r == c ? 1.0 : 0.0;
+            }
+        }
+        cp_async_commit();
+    };
+    fetch_a(first);
+    for (long long i = first; i <= last; ++i) {
+        const long long t = i - first;
+        const bool has_next = !seq || (i < g.N - 1);
+        if (t > 0 && tid == 0) c64_wait1(cx.bM, cx.abort);
+        cp_async_wait_all();
+        __syncthreads();
+        if (*cx.abort) break;
+        // ---- S = A_i - W^T W in sS (its upper triangle) by the slot 0 rows, Z_i into sX by the slot 1 rows
+        if (t > 0) {
+            tc_fence_after();
+            if (live) {
+                const int er = slot == 0 ? ex0[m] : ex1[m];
+                const int rmax = 16 * (w & 3) + 15;  // the last column of S in this warp
+#pragma unroll 1
+                for (int q0 = c0; q0 < c0 + HC; q0 += 8) {
+                    if (seq && q0 > rmax) break;
+                    double v[8];
+                    sl_read8<NB>(tl + (uint32_t)q0, er, ex0 + q0, v);
+                    if (slot == 0) {
+                        if (q0 <= rmax) {
+                            double2 *s = reinterpret_cast<double2 *>(sS + q0 + m * LD);
+#pragma unroll
+                            for (int q = 0; q < 4; ++q) {
+                                double2 x = s[q];
+                                x.x -= v[2 * q];
+                                x.y -= v[2 * q + 1];
+                                s[q] = x;
+                            }
+                        }
+                    } else if (!seq) {
+                        double2 *z = reinterpret_cast<double2 *>(sX + q0 + m * LD);
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) z[q] = make_double2(-v[2 * q], -v[2 * q + 1]);
+                    }
+                }
+            }
+            tc_fence_before();
+            __syncthreads();
+            if (!seq) issue_pl();
+        }
+        // ---- Cholesky + inverse; beside the first pivot tile S_LL, beside the
+        // second one the digits of Z_i (slot 0; first block: B_sL^T) and B_i (slot 1)
+        auto aside = [&](int K) {
+            if (K == 0) {
+                if (t > 0 && !seq && w >= 4) add_sll(t > 1);
+            } else if (K == 1 && w % 4 != 0) {
+                for (int u = w - 1 - w / 4; u < 2 * (NB / 8); u += NW - NW / 4) {
+                    const int gi = u >> 1, row = 8 * gi + (lane & 7);
+                    unsigned char *dst = OP + (uint32_t)(2 * gi + (u & 1)) * G::GRP;
+                    const int valid = row < n ? n : 0;
+                    if ((u & 1) && has_next)
+                        sl_cut_group<NB>(dst, G::SLICE, ex1 + 8 * gi, g.B_in + i * nn + (long long)row * n, 1, valid);
+                    else if (!(u & 1) && !seq && t > 0)
+                        sl_cut_group<NB>(dst, G::SLICE, ex0 + 8 * gi, sX + row * LD, 1, NB);
+                    else if (!(u & 1) && !seq)
+                        sl_cut_group<NB>(dst, G::SLICE, ex0 + 8 * gi, g.B_in + sL * nn + row, n, valid);
+                }
+            }
+        };
+        const int bad = f64_chol_inv_i<NB, SL_THREADS>(sS, sV, sflag, tid, aside);
+        if (bad && tid == 0) record_bad_pivot(g.st, g.level, i);
+        if (*cx.abort) break;
+        // ---- V_i's digits over sS and sX, V_i to global memory while P2 = [Z_i | B_i]^T V_i runs
+        if (has_next) {
+            if (w < NB / 8) sl_cut_group<NB>(OV + (uint32_t)w * G::GRP, G::VSLICE, exV + 8 * w, sV + (8 * w + (lane & 7)) * LD, 1, NB);
+            tc_fence_before();
+            __syncthreads();
+            if (tid == 0) {
+                tc_fence_after();
+                sl_mma<NB>(cx.tm, aOP, aOV, G::GRP);
+                tc_commit(cx.bM.addr);
+                cx.bM.pending = true;
+            }
+        }
+        if (w > 0 || !has_next) {
+            double *dst = g.A_f + i * nn;
+            const int nn32 = n * n;
+            for (int e = has_next ? tid - 32 : tid; e < nn32; e += has_next ? SL_THREADS - 32 : SL_THREADS) {
+                const int c = e / n, r = e - c * n;
+                dst[e] = sV[r + c * LD];
+            }
+        }
+        if (!has_next) break;  // the last block of the sequential chain
+        if (tid == 0) c64_wait1(cx.bM, cx.abort);
+        __syncthreads();
+        if (*cx.abort) break;
+        tc_fence_after();
+        // ---- Y_i (slot 0 rows) and W_i (slot 1 rows) in FP64 over sX and sS
+        if (live) {
+            const int er = slot == 0 ? ex0[m] : ex1[m];
+            double *o = (slot == 0 ? sX : sS) + m * LD;
+#pragma unroll 1
+            for (int q0 = c0; q0 < c0 + HC; q0 += 8) {
+                double v[8];
+                sl_read8<NB>(tl + (uint32_t)q0, er, exV + q0, v);
+#pragma unroll
+                for (int q = 0; q < 8; q += 2) *reinterpret_cast<double2 *>(o + q0 + q) = make_double2(v[q], v[q + 1]);
+            }
+        }
+        tc_fence_before();
+        __syncthreads();
+        // ---- their digits into the slots as [W_i | Y_i]; P1 of the next step (or of the chain end)
+        for (int u = w; u < 2 * (NB / 8); u += NW) {
+            const int gi = u >> 1, row = 8 * gi + (lane & 7);
+            unsigned char *dst = OP + (uint32_t)(2 * gi + (u & 1)) * G::GRP;
+            if (u & 1) {
+                if (!seq) sl_cut_group<NB>(dst, G::SLICE, ex1 + 8 * gi, sX + row * LD, 1, NB);
+            } else {
+                sl_cut_group<NB>(dst, G::SLICE, ex0 + 8 * gi, sS + row * LD, 1, NB);
+            }
+        }
+        __syncthreads();
+        if (tid == 0) {
+            tc_fence_after();
+            sl_mma<NB>(cx.tm, aOP, aOP, 2 * G::GRP);
+            tc_commit(cx.bM.addr);
+            cx.bM.pending = true;
+        } else if (w > 0) {  // meanwhile Y_i and W_i to global memory
+            double *dW = g.B_f + i * nn, *dY = seq ? nullptr : g.Y + i * nn;
+            const int nn32 = n * n;
+            for (int e = tid - 32; e < nn32; e += SL_THREADS - 32) {
+                const int c = e / n, r = e - c * n;
+                dW[e] = sS[r + c * LD];
+                if (!seq) dY[e] = sX[r + c * LD];
+            }
+            asm volatile("bar.sync 2, 224;" ::: "memory");  // sS is read (warp 0 only issues P1)
+            if (i < last) fetch_a(i + 1);
+        }
+    }
+
+    // ---- chain end: S_RR = W^T W, S_LR = Y^T W, the last S_LL term
+    if (!seq && !*cx.abort) {
+        if (tid == 0) c64_wait1(cx.bM, cx.abort);
+        __syncthreads();
+        if (!*cx.abort) {
+            tc_fence_after();
+            if (live) {
+                const int er = slot == 0 ? ex0[m] : ex1[m];
+                double *dst = Cp + (slot == 0 ? nn : 2 * nn);
+#pragma unroll 1
+                for (int q0 = c0; q0 < c0 + HC; q0 += 8) {
+                    double v[8];
+                    sl_read8<NB>(tl + (uint32_t)q0, er, ex0 + q0, v);
+                    if (m < n) {
+#pragma unroll
+                        for (int q = 0; q < 8; ++q)
+                            if (q0 + q < n) dst[m + (long long)(q0 + q) * n] = v[q];
+                    }
+                }
+            }
+            tc_fence_before();
+            __syncthreads();
+            issue_pl();
+            if (w >= 4) add_sll(last > first);
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (*cx.abort) {
+        // a wait gave up: wait (bounded) for the MMAs still in flight before
+        // shared memory and TMEM are released
+        int ignored = 0;
+        if (tid == 0) {
+            c64_wait1(cx.bM, &ignored);
+            if (g.st) atomicExch(&g.st->tc_timeout, 1);
+        } else if (tid == 128) {
+            c64_wait1(cx.bL, &ignored);
+        }
+        __syncthreads();
+    }
+}
+
+template <int NB>
+__device__ __forceinline__ void sl_begin(SlCtx &cx)
+{
+    using G = SlGeo<NB>;
+    extern __shared__ __align__(128) unsigned char smem_sl[];
+    unsigned char *ctl = smem_sl + G::OFF_CTL;
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(ctl + 4);
+    cx.abort = reinterpret_cast<int *>(ctl + 8);
+    uint64_t *mbars = reinterpret_cast<uint64_t *>(ctl + 16);
+    if (threadIdx.x < 32) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
+                     "r"(G::TMEM)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (threadIdx.x == 0) {
+        for (int q = 0; q < 2; ++q)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&mbars[q])) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        *cx.abort = 0;
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    cx.tm = *tslot;
+    cx.bM = C64Bar{smem_u32(&mbars[0]), 0u, false};
+    cx.bL = C64Bar{smem_u32(&mbars[1]), 0u, false};
+}
+
+template <int NB>
+__device__ __forceinline__ void sl_end(const SlCtx &cx)
+{
+    tc_fence_before();
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(cx.tm), "r"(SlGeo<NB>::TMEM)
+                     : "memory");
+    }
+}
+
+template <int NB>
+__global__ void __launch_bounds__(SL_THREADS, NB == 64 ? 1 : 2) chain_f64_tc_kernel(ChainFactorArgs<double, double> g)
+{
+    SlCtx cx;
+    sl_begin<NB>(cx);
+    chain_f64_tc_body<NB>(g, blockIdx.x, cx);
+    sl_end<NB>(cx);
+}
+
+}  // namespace bss

@@ -12,9 +12,10 @@
 //   * pivot tiles (16 x 16, one warp): in-place Gauss-Jordan on [S | I], so
 //     the tile's factor and its inverse come out of one sweep with all 16
 //     column slots always in use: S = L D L^T, V = L^-T D^-1/2.  A pivot
-//     costs 4 + (rows below) / 2 warp-instructions; its reciprocal is an
-//     FP32 seed and one third-order correction (below) instead of a square
-//     root and a division, and the 16 square roots are taken together.
+//     costs 1 + (rows below) / 2 FP64 warp-instructions; its reciprocal is an
+//     FP32 seed and one third-order correction in integers (below) instead of
+//     a square root and a division, runs under the FMAs of the rows that do
+//     not hold the next pivot, and the 16 square roots are taken together.
 //   * row panels U(K, J) = V_KK^T S(K, J), trailing updates and V's
 //     off-diagonal columns: one output per lane, rows grouped so that the
 //     triangular contractions of a warp have (almost) one length.
@@ -50,14 +51,25 @@ __device__ __forceinline__ bool f64_pivot_ordinary(double p)
     return (unsigned)(__double2hiint(p) - (24 << 20)) < (unsigned)(1999 << 20);
 }
 
-// FP32 seed of 1/p for an ordinary p
-__device__ __forceinline__ double f64_rcp_seed(double p)
+// 1/p for an ordinary p, in integer arithmetic (the FP64 port stays free):
+// p = M 2^(E - 1075), the FP32 seed y = Y 2^-24 of the mantissa m = M 2^-52;
+// e = 1 - m y = D 2^-76 with D = -(M Y mod 2^64), then y (1 + e + e^2) in units
+// of 2^-56, rounded once
+__device__ __forceinline__ double f64_rcp(double p)
 {
     const unsigned hi = (unsigned)__double2hiint(p), lo = (unsigned)__double2loint(p);
-    const float m = __uint_as_float(0x3F800000u | ((hi & 0xFFFFFu) << 3) | (lo >> 29));
+    const unsigned mh = (hi & 0xFFFFFu) | 0x100000u;
     float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(m));
-    return f64_from_seed(y, (int)(hi >> 20) - 1023);
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(__uint_as_float(0x3F800000u | ((hi & 0xFFFFFu) << 3) | (lo >> 29))));
+    const unsigned yb = __float_as_uint(y);
+    const unsigned Y = ((yb & 0x7FFFFFu) | 0x800000u) << ((yb >> 23) - 126u);  // y in (1/2, 1]
+    const unsigned long long MY = (unsigned long long)lo * Y + ((unsigned long long)(mh * Y) << 32);
+    const long long D = (long long)(0ull - MY);
+    const int es = (int)(D >> 32);
+    const long long t = (D >> 20) + __mulhi(es, es);  // e + e^2 in units of 2^-56
+    const long long Yt = (long long)((unsigned long long)(unsigned)t * Y + ((unsigned long long)((unsigned)(t >> 32) * Y) << 32));
+    const unsigned long long R = ((unsigned long long)Y << 32) + (unsigned long long)(Yt >> 24);
+    return __longlong_as_double((long long)(((R + 4) >> 3) + ((unsigned long long)(1021u + 1023u - (hi >> 20)) << 52)));
 }
 
 // 1/sqrt(p), p > 0
@@ -90,18 +102,18 @@ __device__ __forceinline__ int f64_pivot_tile(const double *sS, double *sV, int 
     }
     int bad = 0;
     double dj = 1.0;
+    double piv = __shfl_sync(ALL, v[0], 0);
+    double row = __shfl_sync(ALL, v[0], c);  // row j: S right of the pivot, L^-1 left of it
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
         const int hj = j & 1, qj = j >> 1;
-        double piv = __shfl_sync(ALL, v[qj], j + 16 * hj);
-        double row = __shfl_sync(ALL, v[qj], c + 16 * hj);  // row j: S right of the pivot, L^-1 left of it
         if (c == j) row = 1.0;
+        double s[8];  // S(j, row q of this lane)
+#pragma unroll
+        for (int q = (j + 1) >> 1; q < 8; ++q) s[q] = __shfl_sync(ALL, v[qj], 2 * q + h + 16 * hj);
         double m;  // row / pivot
         if (f64_pivot_ordinary(piv)) {
-            const double y = f64_rcp_seed(piv);
-            const double w = row * y;
-            const double e = fma(-piv, y, 1.0);
-            m = fma(w, fma(e, e, e), w);
+            m = row * f64_rcp(piv);
         } else {
             if (!(piv > 0.0 && piv < INFINITY)) {
                 bad = 1;
@@ -110,12 +122,16 @@ __device__ __forceinline__ int f64_pivot_tile(const double *sS, double *sV, int 
             m = row / piv;
         }
         if (c == j) dj = piv;
+        // row j + 1 first: the next pivot's broadcasts and reciprocal run under the other rows' FMAs
 #pragma unroll
         for (int q = (j + 1) >> 1; q < 8; ++q) {
-            const double s = __shfl_sync(ALL, v[qj], 2 * q + h + 16 * hj);  // S(j, row of this lane)
             const double base = c == j ? 0.0 : v[q];
-            const double x = fma(-s, m, base);
+            const double x = fma(-s[q], m, base);
             if (2 * q > j || h == 1) v[q] = x;  // the first q of an even j also holds the pivot row (h = 0)
+            if (q == (j + 1) >> 1) {
+                piv = __shfl_sync(ALL, v[q], (j + 1) + 16 * (hj ^ 1));
+                row = __shfl_sync(ALL, v[q], c + 16 * (hj ^ 1));
+            }
         }
     }
     const double rs = f64_rsqrt(dj);
@@ -242,23 +258,32 @@ __device__ __forceinline__ constexpr int f64_aside()
     return NW - (NW + 3) / 4;
 }
 
-template <int LD, int NW, int NB, int K>
-__device__ __forceinline__ void f64_chol_panel(double *sS, double *sV, int *sflag, int warp, int lane)
+// `aside(K)` runs on the warps other than warp 0 while that factors pivot tile
+// K: the caller's own work, which must not touch sS or sV.
+struct F64NoAside {
+    __device__ __forceinline__ void operator()(int) const {}
+};
+
+template <int LD, int NW, int NB, int K, class Aside>
+__device__ __forceinline__ void f64_chol_panel(double *sS, double *sV, int *sflag, int warp, int lane, Aside &aside)
 {
     constexpr int KP = NB / 16, o = 16 * K;
     constexpr int NA = f64_aside<NW>();
     if (warp == 0) {
         const int bad = f64_pivot_tile<LD>(sS, sV, o, lane);
         if (bad && lane == 0) *sflag = 1;
-    } else if constexpr (K >= 2) {
-        if (warp % 4 != 0) f64_inv_column<LD, NA, K - 1>(sS, sV, warp - 1 - warp / 4, lane, 1);
+    } else {
+        aside(K);
+        if constexpr (K >= 2) {
+            if (warp % 4 != 0) f64_inv_column<LD, NA, K - 1>(sS, sV, warp - 1 - warp / 4, lane, 1);
+        }
     }
     __syncthreads();
     if constexpr (K + 1 < KP) {
         f64_row_panel<LD, NW, KP - 1 - K>(sS, sV, o, warp, lane);
         f64_trailing<LD, 32 * NW, NB - o - 16>(sS, o, 32 * warp + lane);
         __syncthreads();
-        f64_chol_panel<LD, NW, NB, K + 1>(sS, sV, sflag, warp, lane);
+        f64_chol_panel<LD, NW, NB, K + 1>(sS, sV, sflag, warp, lane, aside);
     } else if constexpr (KP > 1) {
         f64_inv_column<LD, NW, KP - 1>(sS, sV, warp, lane, 0);
         __syncthreads();
@@ -266,12 +291,18 @@ __device__ __forceinline__ void f64_chol_panel(double *sS, double *sV, int *sfla
 }
 
 // the whole tile (contract of chol_inv_blocked; sS keeps no factor)
+template <int NB, int THREADS, class Aside>
+__device__ __forceinline__ int f64_chol_inv_i(double *sS, double *sV, int *sflag, int tid, Aside &aside)
+{
+    if (tid == 0) *sflag = 0;  // (set by the same thread: no barrier needed before it)
+    f64_chol_panel<Geo<double, NB>::LD, THREADS / 32, NB, 0>(sS, sV, sflag, tid >> 5, tid & 31, aside);
+    return *sflag;
+}
 template <int NB, int THREADS>
 __device__ __noinline__ int f64_chol_inv(double *sS, double *sV, int *sflag, int tid)
 {
-    if (tid == 0) *sflag = 0;  // (set by the same thread: no barrier needed before it)
-    f64_chol_panel<Geo<double, NB>::LD, THREADS / 32, NB, 0>(sS, sV, sflag, tid >> 5, tid & 31);
-    return *sflag;
+    F64NoAside none;
+    return f64_chol_inv_i<NB, THREADS>(sS, sV, sflag, tid, none);
 }
 
 }  // namespace bss

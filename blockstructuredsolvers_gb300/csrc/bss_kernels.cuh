@@ -3017,5 +3017,6 @@ __global__ void init_identity_kernel(T *A, long long first_blk, long long last_b
 }  // namespace bss
 
 #include "bss_chain64_tc.cuh"
+#include "bss_chain_f64_tc.cuh"
 #include "bss_chain128_tc.cuh"
 #include "bss_stream.cuh"

@@ -30,12 +30,31 @@ static cudaError_t chain64_tc(const ChainFactorArgs<Tin, float> &a, cudaStream_t
     return cudaGetLastError();
 }
 
+// FP64 chains of 17..64-wide blocks: products on the tensor cores by digits
+// (bss_chain_f64_tc.cuh).  Up to 16 a block's products are 128 full FP64
+// warp-instructions each (2.4K cycles an SM), about what cutting and putting
+// together the digits would take, and the FP64-pipe kernel stays.
+template <int NB>
+static cudaError_t chain_f64_tc(const ChainFactorArgs<double, double> &a, cudaStream_t s)
+{
+    auto kern = chain_f64_tc_kernel<NB>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SlGeo<NB>::BYTES);
+    if (e != cudaSuccess) return e;
+    cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    kern<<<a.seq ? 1u : (unsigned)a.Q, SL_THREADS, SlGeo<NB>::BYTES, s>>>(a);
+    count_launch();
+    return cudaGetLastError();
+}
+
 template <class Tin, class T, int NB>
 static cudaError_t chain_factor_nb(const ChainFactorArgs<Tin, T> &a, cudaStream_t s)
 {
     if constexpr (std::is_same<T, float>::value && NB == 64) {
         if (!a.seq && !(a.variant & FACTOR_FMA_CHAIN)) return chain64_tc<Tin>(a, s);
     }
+    if constexpr (std::is_same<T, double>::value && NB >= 32) {
+        return chain_f64_tc<NB>(a, s);
+    } else {
     const size_t smem = chain_factor_smem<T, NB>();
     auto kern = chain_factor_kernel<Tin, T, NB>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -44,6 +63,7 @@ static cudaError_t chain_factor_nb(const ChainFactorArgs<Tin, T> &a, cudaStream_
     kern<<<grid, Tile<NB>::THREADS, smem, s>>>(a);
     count_launch();
     return cudaGetLastError();
+    }
 }
 
 template <class Tin, class T, bool TC>
@@ -156,6 +176,9 @@ static int ctas_nb(int variant)
             cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
             return ctas_per_sm(kern, C64_THREADS, smem);
         }
+    }
+    if constexpr (std::is_same<T, double>::value && NB >= 32) {
+        return NB == 64 ? 1 : 2;  // by shared memory and TMEM; by registers and TMEM
     }
     const size_t smem = chain_factor_smem<T, NB>();
     auto kern = chain_factor_kernel<Tin, T, NB>;

@@ -40,8 +40,10 @@
 //
 // Measured (the digit products of one operand pair: 4.7K cycles for NB = 64,
 // 1.4K for NB = 32, against 131K and 16K for one product on the FP64 pipe):
-// plain FP64 factor + solve of N = 16384, n = 64: 35.6 -> 13.3 ms; N = 1531,
-// n = 37, k = 3: 6.42 -> 2.77 ms; N = 100, n = 32: 679 -> 476 us.
+// plain FP64 factor + solve of N = 16384, n = 64: 35.6 -> 11.3 ms; N = 1531,
+// n = 37, k = 3: 6.42 -> 2.68 ms; N = 100, n = 32: 679 -> 435 us.  A 64-wide step
+// takes ~145K cycles: 49K in the four pivot tiles, 46K in the Cholesky's other
+// FP64 products, 31K cutting and putting together digits, 15K in MMAs.
 #pragma once
 
 namespace bss {
@@ -59,8 +61,8 @@ struct SlGeo {
     static constexpr uint32_t OFF_S = SL_DIGITS * SLICE;         // sS; after the Cholesky sS and X hold the V operand
     static constexpr uint32_t OFF_X = OFF_S + TILE;              // Z in FP64; after P2 (sS, sX) hold W and Y in FP64
     static constexpr uint32_t OFF_V = OFF_X + TILE;              // sV
-    static constexpr uint32_t OFF_EX = OFF_V + TILE;             // row exponents: slot 0, slot 1, V
-    static constexpr uint32_t OFF_CTL = OFF_EX + 3u * 64u * 4u;
+    static constexpr uint32_t OFF_EX = OFF_V + TILE;             // row exponents: slot 0 (W, Z), Y, B (slot 1), V
+    static constexpr uint32_t OFF_CTL = OFF_EX + 4u * 64u * 4u;
     static constexpr uint32_t BYTES = OFF_CTL + 64u;
     static constexpr uint32_t TMEM = SL_LEVELS * NB;
     static_assert(SL_DIGITS * VSLICE <= 2 * TILE, "the V operand overlays sS and X");
@@ -119,25 +121,47 @@ __device__ __forceinline__ void sl_mma(uint32_t tm, uint32_t a, uint32_t b, uint
     }
 }
 
-// value v 2^e as FP64 (one rounding, to nearest); NaN for the marked exponents
-__device__ __forceinline__ double sl_to_f64(long long v, int e)
+// value v 2^e as FP64, in full: subnormal and infinite results, NaN for the
+// marked exponents
+static __device__ __noinline__ double sl_to_f64_rare(long long v, int e)
 {
-    const unsigned long long u0 = (unsigned long long)(v < 0 ? -v : v);
-    const unsigned uh = (unsigned)(u0 >> 32), ul = (unsigned)u0;
-    const int lz = uh ? __clz((int)uh) : 32 + __clz((int)ul);
-    const unsigned long long u = u0 << (lz & 63);
-    const unsigned long long q = (u >> 11) + ((u >> 10) & 1ull);  // 53 bits, the top one set
-    const int be = e + 63 - lz + 1023;
-    unsigned long long bits = ((unsigned long long)(unsigned)(be - 1) << 52) + q;
-    if (be <= 0) {  // subnormal
-        const int s = 12 - be;
-        bits = s > 63 ? 0ull : (u >> s) + ((u >> (s - 1)) & 1ull);
+    if (e >= SL_NAN / 2) return __longlong_as_double(0x7FF8000000000000ll);
+    const unsigned long long u0 = (unsigned long long)(v < 0 ? ~v : v);
+    unsigned long long bits = 0;
+    if (u0 != 0) {
+        const int lz = __clzll((long long)u0), be = e + 63 - lz + 1023;
+        const unsigned long long u = u0 << lz;
+        if (be >= 2047)
+            bits = 0x7FF0000000000000ull;
+        else if (be > 0)
+            bits = ((unsigned long long)(be - 1) << 52) + (u >> 11) + ((u >> 10) & 1ull);
+        else if (be > -52)
+            bits = (u >> (12 - be)) + ((u >> (11 - be)) & 1ull);
     }
-    if (be >= 2047) bits = 0x7FF0000000000000ull;
-    if (u0 == 0) bits = 0;
-    if (v < 0) bits |= 0x8000000000000000ull;
-    if (e >= SL_NAN / 2) bits = 0x7FF8000000000000ull;
-    return __longlong_as_double((long long)bits);
+    return __longlong_as_double((long long)(bits | (v < 0 ? 0x8000000000000000ull : 0ull)));
+}
+// the same for ordinary results, one rounding to nearest (|v| of a negative v
+// is taken one unit, 2^-56 of the scale, small); sets `rare` where the above
+// has to be asked instead.  32-bit operations spelled out (64-bit shifts by a
+// variable compile to three times as many) and no branch, so that a thread's
+// elements overlap: integer instructions run at half rate here and this is
+// what a readout spends its time on.
+__device__ __forceinline__ double sl_to_f64(long long v, int e, bool &rare)
+{
+    const unsigned vh = (unsigned)((unsigned long long)v >> 32), sg = (unsigned)((int)vh >> 31);
+    const unsigned uh = vh ^ sg, ul = (unsigned)v ^ sg;
+    const bool low = uh == 0;
+    const unsigned h = low ? ul : uh, l = low ? 0u : ul;
+    const int lz = __clz((int)h);
+    const unsigned mh = __funnelshift_l(l, h, lz), ml = l << (lz & 31);  // bit 31 of mh set (h != 0)
+    const int be1 = e + 63 + 1022 - lz - (low ? 32 : 0);                 // biased exponent - 1
+    rare |= (unsigned)be1 > 2045u;  // (zeros too where the exponents are far down or marked)
+    const unsigned ql = __funnelshift_r(ml, mh, 11), r = (ml >> 10) & 1u;
+    unsigned lo, hi;
+    asm("add.cc.u32 %0, %2, %3;\n addc.u32 %1, %4, %5;" : "=r"(lo), "=r"(hi) : "r"(ql), "r"(r), "r"(mh >> 11), "r"((unsigned)be1 << 20));
+    lo = h ? lo : 0u;
+    hi = h ? (hi | (sg & 0x80000000u)) : 0u;
+    return __hiloint2double((int)hi, (int)lo);
 }
 
 // eight accumulator columns of this thread's TMEM lane, all levels -> FP64:
@@ -159,6 +183,8 @@ __device__ __forceinline__ void sl_read8(uint32_t addr, int er, const int *ec, d
     // conversion instruction takes ~30 cycles of a scheduler, an add one.
     constexpr float C23 = 12582912.f, C24 = 25165824.f;
     constexpr unsigned B23 = 0x4B400000u, B24 = 0x4BC00000u;
+    bool rare = false;
+    long long vs[8];
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
         unsigned b[SL_LEVELS];
@@ -177,8 +203,12 @@ __device__ __forceinline__ void sl_read8(uint32_t addr, int er, const int *ec, d
         const int t2 = (int)(b[4] * 256u + b[5] - (B23 * 256u + 2u * B24 + B23));
         const int t3 = (int)(b[6] * 256u + b[7] - (B23 * 256u + B23));  // halved
         // unit 2^-56 (level l has unit 2^-(12 + 8 l)); |v| <= 2^62
-        const long long v = (long long)((unsigned long long)(long long)t0 << 36) + (long long)t1 * (1 << 20) + (long long)t2 * 16 + (t3 >> 11);
-        out[q] = sl_to_f64(v, er + ec[q] - 56);
+        vs[q] = (long long)((unsigned long long)(long long)t0 << 36) + (long long)t1 * (1 << 20) + (long long)t2 * 16 + (t3 >> 11);
+        out[q] = sl_to_f64(vs[q], er + ec[q] - 56, rare);
+    }
+    if (rare) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) out[q] = sl_to_f64_rare(vs[q], er + ec[q] - 56);
     }
 }
 
@@ -197,12 +227,22 @@ __device__ __forceinline__ void sl_put8(unsigned char *dst, uint32_t stride, con
         const int E = (int)((xh >> 20) & 0x7FFu);
         const unsigned mh = (xh & 0xFFFFFu) | (E ? 0x100000u : 0u);
         int sh = emax - (E ? E : 1);
-        sh = sh > 63 ? 63 : sh;
-        unsigned long long m = (((unsigned long long)mh << 32) | xl) << 2;
-        m = ((m >> sh) + 1) >> 1;  // |x| 2^54 / 2^(row exponent), rounded
-        const unsigned long long b = ((xh >> 31) ? 0ull - m : m) + 0x0080808080808080ull;  // byte 6 - s = digit s + 128
-        lo[q] = (uint32_t)b;
-        hi[q] = (uint32_t)(b >> 32);
+        // |x| 2^54 / 2^(row exponent), rounded: ((M << 2) >> sh) + 1 >> 1
+        const unsigned h0 = __funnelshift_l(xl, mh, 2), l0 = xl << 2;
+        const bool far = sh >= 32;
+        sh = min(sh, 63);
+        unsigned h = far ? 0u : h0, l = far ? h0 : l0;
+        l = __funnelshift_r(l, h, sh);  // (by sh % 32; h0 < 2^23, so a shift by 31 leaves nothing of it)
+        h >>= (sh & 31);
+        unsigned r0, r1;
+        asm("add.cc.u32 %0, %2, 1;\n addc.u32 %1, %3, 0;" : "=r"(r0), "=r"(r1) : "r"(l), "r"(h));
+        r0 = __funnelshift_r(r0, r1, 1);
+        r1 >>= 1;
+        const unsigned sg = (unsigned)((int)xh >> 31);
+        // byte 6 - s = digit s + 128: (|x| ^ sg) - sg + 0x0080808080808080
+        asm("add.cc.u32 %0, %2, %4;\n addc.u32 %1, %3, %5;"
+            : "=r"(lo[q]), "=r"(hi[q])
+            : "r"(r0 ^ sg), "r"(r1 ^ sg), "r"(0x80808080u - sg), "r"(0x00808080u));
     }
 #pragma unroll
     for (int s = 0; s < SL_DIGITS; ++s) {
@@ -268,7 +308,7 @@ __device__ __forceinline__ void chain_f64_tc_body(const ChainFactorArgs<double, 
     double *sX = reinterpret_cast<double *>(smem_sl + G::OFF_X);
     double *sV = reinterpret_cast<double *>(smem_sl + G::OFF_V);
     unsigned char *OV = smem_sl + G::OFF_S;                        // the V operand
-    int *ex0 = reinterpret_cast<int *>(smem_sl + G::OFF_EX), *ex1 = ex0 + 64, *exV = ex1 + 64;
+    int *ex0 = reinterpret_cast<int *>(smem_sl + G::OFF_EX), *ex1 = ex0 + 64, *exB = ex1 + 64, *exV = exB + 64;
     int *sflag = reinterpret_cast<int *>(smem_sl + G::OFF_CTL);
     const uint32_t aOP = smem_u32(OP), aOV = smem_u32(OV);
 
@@ -295,24 +335,26 @@ __device__ __forceinline__ void chain_f64_tc_body(const ChainFactorArgs<double, 
     for (int e = tid; e < Geo<double, NB>::SLOT; e += SL_THREADS) sV[e] = 0.0;  // V's strictly lower tiles stay zero
     __syncthreads();
 
-    // S_LL (+)= Y^T Y from the PL accumulator, by warps 4-7 (named barrier 3)
-    auto add_sll = [&](bool add) {
+    // S_LL (+)= Y^T Y from the PL accumulator: its columns qa .. qb - 1, by warps 4-7
+    auto wait_pl = [&]() {  // warps 1-7
         if (tid == 128) c64_wait1(cx.bL, cx.abort);
-        asm volatile("bar.sync 3, 128;" ::: "memory");
+        asm volatile("bar.sync 3, 224;" ::: "memory");
+    };
+    auto add_sll = [&](bool add, int qa, int qb) {
         if (*cx.abort || !live) return;
         tc_fence_after();
         const int er = ex1[m];
 #pragma unroll 1
-        for (int q0 = 0; q0 < NB; q0 += 8) {
+        for (int q0 = qa; q0 < qb; q0 += 8) {
             double v[8];
             sl_read8<NB>(tl + (uint32_t)q0, er, ex1 + q0, v);
             if (slot == 1 && m < n) {
+                double c[8];
+#pragma unroll
+                for (int q = 0; q < 8; ++q) c[q] = add && q0 + q < n ? __ldcg(Cp + m + (long long)(q0 + q) * n) : 0.0;
 #pragma unroll
                 for (int q = 0; q < 8; ++q)
-                    if (q0 + q < n) {
-                        double *c = Cp + m + (long long)(q0 + q) * n;
-                        *c = add ? *c + v[q] : v[q];
-                    }
+                    if (q0 + q < n) __stcg(Cp + m + (long long)(q0 + q) * n, c[q] + v[q]);
             }
         }
         tc_fence_before();
@@ -385,21 +427,23 @@ __device__ __forceinline__ void chain_f64_tc_body(const ChainFactorArgs<double, 
             __syncthreads();
             if (!seq) issue_pl();
         }
-        // ---- Cholesky + inverse; beside the first pivot tile S_LL, beside the
-        // second one the digits of Z_i (slot 0; first block: B_sL^T) and B_i (slot 1)
+        // ---- Cholesky + inverse; beside the first two pivot tiles S_LL (warps 4-7) and
+        // the digits of B_i (slot 1) and Z_i (slot 0; first block: B_sL^T) (warps 1-3)
         auto aside = [&](int K) {
-            if (K == 0) {
-                if (t > 0 && !seq && w >= 4) add_sll(t > 1);
-            } else if (K == 1 && w % 4 != 0) {
-                for (int u = w - 1 - w / 4; u < 2 * (NB / 8); u += NW - NW / 4) {
-                    const int gi = u >> 1, row = 8 * gi + (lane & 7);
-                    unsigned char *dst = OP + (uint32_t)(2 * gi + (u & 1)) * G::GRP;
-                    const int valid = row < n ? n : 0;
-                    if ((u & 1) && has_next)
-                        sl_cut_group<NB>(dst, G::SLICE, ex1 + 8 * gi, g.B_in + i * nn + (long long)row * n, 1, valid);
-                    else if (!(u & 1) && !seq && t > 0)
+            const bool pl = t > 0 && !seq;
+            if (K == 0 && pl) wait_pl();
+            if (K <= 1 && w >= 4) {
+                constexpr int PART = (5 * NB / 8 + 7) / 8 * 8;  // most of them beside the first, which starts late
+                if (pl) add_sll(t > 1, K == 0 ? 0 : PART, K == 0 ? PART : NB);
+            } else if (K <= 1) {
+                for (int gi = w - 1; gi < NB / 8; gi += 3) {
+                    const int row = 8 * gi + (lane & 7), valid = row < n ? n : 0;
+                    unsigned char *dst = OP + (uint32_t)(2 * gi + 1 - K) * G::GRP;
+                    if (K == 0 && has_next)
+                        sl_cut_group<NB>(dst, G::SLICE, exB + 8 * gi, g.B_in + i * nn + (long long)row * n, 1, valid);
+                    else if (K == 1 && pl)
                         sl_cut_group<NB>(dst, G::SLICE, ex0 + 8 * gi, sX + row * LD, 1, NB);
-                    else if (!(u & 1) && !seq)
+                    else if (K == 1 && !seq)
                         sl_cut_group<NB>(dst, G::SLICE, ex0 + 8 * gi, g.B_in + sL * nn + row, n, valid);
                 }
             }
@@ -434,7 +478,7 @@ __device__ __forceinline__ void chain_f64_tc_body(const ChainFactorArgs<double, 
         tc_fence_after();
         // ---- Y_i (slot 0 rows) and W_i (slot 1 rows) in FP64 over sX and sS
         if (live) {
-            const int er = slot == 0 ? ex0[m] : ex1[m];
+            const int er = slot == 0 ? ex0[m] : exB[m];
             double *o = (slot == 0 ? sX : sS) + m * LD;
 #pragma unroll 1
             for (int q0 = c0; q0 < c0 + HC; q0 += 8) {
@@ -498,7 +542,8 @@ __device__ __forceinline__ void chain_f64_tc_body(const ChainFactorArgs<double, 
             tc_fence_before();
             __syncthreads();
             issue_pl();
-            if (w >= 4) add_sll(last > first);
+            if (w > 0) wait_pl();
+            if (w >= 4) add_sll(last > first, 0, NB);
         }
     }
     tc_fence_before();

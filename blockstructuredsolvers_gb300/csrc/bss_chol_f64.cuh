@@ -89,8 +89,10 @@ __device__ __forceinline__ double f64_rsqrt(double p)
 // Lane = column slot c (lane % 16) and row parity h (lane / 16); v[q] is row
 // 2 q + h.  Slot c of a row r holds S(r, c) until column c is eliminated and
 // the inverse's L^-1(r, c) from then on.
+// Out of line: 40 KB of straight code that every panel shares (one copy per
+// panel ran 1.5 times as long, on instruction fetches).
 template <int LD>
-__device__ __forceinline__ int f64_pivot_tile(const double *sS, double *sV, int o, int lane)
+__device__ __noinline__ int f64_pivot_tile(const double *sS, double *sV, int o, int lane)
 {
     constexpr unsigned ALL = 0xFFFFFFFFu;
     const int c = lane & 15, h = lane >> 4;

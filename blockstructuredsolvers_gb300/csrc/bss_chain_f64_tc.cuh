@@ -562,18 +562,16 @@ __device__ __forceinline__ void chain_f64_tc_body(const ChainFactorArgs<double, 
     }
 }
 
-template <int NB>
-__device__ __forceinline__ void sl_begin(SlCtx &cx)
+// TMEM columns and mbarriers of a CTA; ctl: 64 bytes (the first word is the
+// Cholesky's flag)
+__device__ __forceinline__ void sl_begin(SlCtx &cx, unsigned char *ctl, uint32_t cols)
 {
-    using G = SlGeo<NB>;
-    extern __shared__ __align__(128) unsigned char smem_sl[];
-    unsigned char *ctl = smem_sl + G::OFF_CTL;
     uint32_t *tslot = reinterpret_cast<uint32_t *>(ctl + 4);
     cx.abort = reinterpret_cast<int *>(ctl + 8);
     uint64_t *mbars = reinterpret_cast<uint64_t *>(ctl + 16);
     if (threadIdx.x < 32) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
-                     "r"(G::TMEM)
+                     "r"(cols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -591,14 +589,13 @@ __device__ __forceinline__ void sl_begin(SlCtx &cx)
     cx.bL = C64Bar{smem_u32(&mbars[1]), 0u, false};
 }
 
-template <int NB>
-__device__ __forceinline__ void sl_end(const SlCtx &cx)
+__device__ __forceinline__ void sl_end(const SlCtx &cx, uint32_t cols)
 {
     tc_fence_before();
     __syncthreads();
     if (threadIdx.x < 32) {
         tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(cx.tm), "r"(SlGeo<NB>::TMEM)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(cx.tm), "r"(cols)
                      : "memory");
     }
 }
@@ -606,10 +603,11 @@ __device__ __forceinline__ void sl_end(const SlCtx &cx)
 template <int NB>
 __global__ void __launch_bounds__(SL_THREADS, NB == 64 ? 1 : 2) chain_f64_tc_kernel(ChainFactorArgs<double, double> g)
 {
+    extern __shared__ __align__(128) unsigned char smem_sl[];
     SlCtx cx;
-    sl_begin<NB>(cx);
+    sl_begin(cx, smem_sl + SlGeo<NB>::OFF_CTL, SlGeo<NB>::TMEM);
     chain_f64_tc_body<NB>(g, blockIdx.x, cx);
-    sl_end<NB>(cx);
+    sl_end(cx, SlGeo<NB>::TMEM);
 }
 
 }  // namespace bss

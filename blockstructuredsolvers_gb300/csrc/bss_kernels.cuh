@@ -3018,5 +3018,6 @@ __global__ void init_identity_kernel(T *A, long long first_blk, long long last_b
 
 #include "bss_chain64_tc.cuh"
 #include "bss_chain_f64_tc.cuh"
+#include "bss_chain128_f64_tc.cuh"
 #include "bss_chain128_tc.cuh"
 #include "bss_stream.cuh"

@@ -142,12 +142,29 @@ static cudaError_t chain128_tc(const ChainFactorArgs<Tin, float> &a, cudaStream_
     return cudaGetLastError();
 }
 
+// FP64 chains of 65..128-wide blocks: tile products on the tensor cores by
+// digits (bss_chain128_f64_tc.cuh); wider blocks keep the FP64 pipe
+template <class T>
+static cudaError_t chain128_f64_tc(const ChainFactorArgs<T, T> &a, cudaStream_t s)
+{
+    auto kern = chain128_f64_tc_kernel<T>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WlGeo::BYTES);
+    if (e != cudaSuccess) return e;
+    cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    kern<<<a.seq ? 1u : (unsigned)a.Q, SL_THREADS, WlGeo::BYTES, s>>>(a);
+    count_launch();
+    return cudaGetLastError();
+}
+
 template <class Tin, class T>
 static cudaError_t wide_chain_factor(const ChainFactorArgs<Tin, T> &a, cudaStream_t s)
 {
     if constexpr (std::is_same<T, float>::value) {
         if (use_chain128<Tin>(a)) return chain128_tc<Tin>(a, s);
         if (wide_uses_tc<T>(a.n)) return wide_chain_factor_tc<Tin, T, true>(a, s);
+    }
+    if constexpr (std::is_same<T, double>::value) {
+        if (a.n <= 128) return chain128_f64_tc<T>(a, s);
     }
     return wide_chain_factor_tc<Tin, T, false>(a, s);
 }
@@ -214,6 +231,7 @@ int chain_factor_ctas_per_sm(int n, int variant)
             if (n <= 128 && !(variant & FACTOR_WIDE_L2)) return 2;
             if (wide_uses_tc<T>(n)) return wide_ctas_tc<Tin, T, true>();
         }
+        if (std::is_same<T, double>::value && n <= 128) return 1;  // chain128_f64_tc: shared memory and TMEM
         return wide_ctas_tc<Tin, T, false>();
     default: return 1;
     }

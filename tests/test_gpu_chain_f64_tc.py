@@ -1,5 +1,5 @@
-"""FP64 chain kernel with digit products on the tensor cores
-(csrc/bss_chain_f64_tc.cuh): both tile sizes and their remainders, chains with
+"""FP64 chain kernels with digit products on the tensor cores
+(csrc/bss_chain_f64_tc.cuh, csrc/bss_chain128_f64_tc.cuh): all tile sizes and their remainders, chains with
 and without separators, rows of very different sizes, and non-finite blocks."""
 import numpy as np
 import pytest
@@ -32,7 +32,7 @@ def _solve(data, N):
 
 
 @pytest.mark.parametrize("parts", [0, 1, 3])
-@pytest.mark.parametrize("n", [17, 24, 31, 32, 33, 40, 49, 63, 64])
+@pytest.mark.parametrize("n", [17, 24, 31, 32, 33, 40, 49, 63, 64, 65, 72, 97, 127, 128])
 def test_against_oracle(n, parts):
     rng = np.random.default_rng(100 * n + parts)
     A, B, d = O.gen_shifted_family(rng, 17, n, 2, diag_shift=2.0 * n, b_scale=0.5)
@@ -40,11 +40,11 @@ def test_against_oracle(n, parts):
     assert O.rel_error(x, cref.solve_math(A, B, d, np.float64)) <= 1e-10
 
 
-@pytest.mark.parametrize("n", [32, 37, 64])
+@pytest.mark.parametrize("n", [32, 37, 64, 70, 128])
 def test_rows_of_different_sizes(n):
     """T -> D T D with D = diag(2^-12 .. 2^12): digits are cut row by row, so every
     row keeps its own precision.  Backward error of a block Cholesky is a small
-    multiple of n u (n = 64: 7e-15): 1e-13 with the widened row norms."""
+    multiple of n u (n = 128: 1.4e-14): 1e-13 with the widened row norms."""
     rng = np.random.default_rng(n)
     A, B, d = O.gen_shifted_family(rng, 19, n, 1, diag_shift=2.0 * n, b_scale=0.5)
     D = 2.0 ** rng.integers(-12, 13, (19, n))
@@ -57,7 +57,7 @@ def test_rows_of_different_sizes(n):
 
 @pytest.mark.parametrize("value", [float("nan"), float("inf")])
 @pytest.mark.parametrize("where", ["A", "B"])
-@pytest.mark.parametrize("n", [32, 64])
+@pytest.mark.parametrize("n", [32, 64, 100])
 def test_non_finite_blocks_are_reported(n, where, value):
     rng = np.random.default_rng(n)
     A, B, d = O.gen_shifted_family(rng, 11, n, 1, diag_shift=2.0 * n, b_scale=0.5)

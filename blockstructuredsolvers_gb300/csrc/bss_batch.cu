@@ -142,6 +142,19 @@ cudaError_t queue_factor_nb(const ChainFactorArgs<Tin, T> *descs, const WorkItem
     return cudaGetLastError();
 }
 
+template <class Tin, class T>
+cudaError_t queue_factor16(const ChainFactorArgs<Tin, T> *descs, const WorkItem *items, int nitems, int *head, int sms,
+                           cudaStream_t s)
+{
+    auto kern = chain16_queue_kernel<Tin, T>;
+    const int grid = std::max(1, std::min(nitems, sms * ctas_per_sm(kern, C16_THREADS, C16Geo<T>::BYTES)));
+    const cudaError_t e = cudaMemsetAsync(head, 0, sizeof(int), s);
+    if (e != cudaSuccess) return e;
+    kern<<<grid, C16_THREADS, C16Geo<T>::BYTES, s>>>(descs, items, nitems, head);
+    count_launch();
+    return cudaGetLastError();
+}
+
 template <class Tin, class T, bool TC>
 cudaError_t queue_factor_wide(const ChainFactorArgs<Tin, T> *descs, const WorkItem *items, int nitems, int *head,
                               int sms, cudaStream_t s)
@@ -168,7 +181,7 @@ cudaError_t queue_factor(int nb, const ChainFactorArgs<Tin, T> *descs, const Wor
     case WIDE_CLASS: return queue_factor_wide<Tin, T, false>(descs, items, nitems, head, sms, s);
     case WIDE_CLASS + 1: return queue_factor_wide<Tin, T, std::is_same<T, float>::value>(descs, items, nitems, head,
                                                                                          sms, s);
-    case 16: return queue_factor_nb<Tin, T, 16>(descs, items, nitems, head, sms, s);
+    case 16: return queue_factor16<Tin, T>(descs, items, nitems, head, sms, s);
     case 32: return queue_factor_nb<Tin, T, 32>(descs, items, nitems, head, sms, s);
     default: return queue_factor_nb<Tin, T, 64>(descs, items, nitems, head, sms, s);
     }

@@ -60,18 +60,32 @@ static __device__ __noinline__ void wl_emit(uint32_t tm, const int *ex, const in
     const double *base = slot ? base1 : base0;
     const bool mine = dst != nullptr && m < (slot ? nr1 : nr0);
     const int er = ex[64 * slot + m];
+    const bool add = mine && base != nullptr;
+    const long long flip = sign < 0.0 ? (long long)0x8000000000000000ull : 0;
     tc_fence_after();
+    double c[8];  // base, fetched one chunk ahead
+#pragma unroll
+    for (int q = 0; q < 8; ++q) c[q] = add && c0 + q < nc ? __ldcg(base + m + (long long)(c0 + q) * n) : 0.0;
 #pragma unroll 1
     for (int q0 = c0; q0 < c0 + 32 && q0 < nc; q0 += 8) {
-        double c[8], v[8];
+        double v[8], cn[8];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) c[q] = mine && base && q0 + q < nc ? __ldcg(base + m + (long long)(q0 + q) * n) : 0.0;
+        for (int q = 0; q < 8; ++q)
+            cn[q] = add && q0 + 8 < c0 + 32 && q0 + 8 + q < nc ? __ldcg(base + m + (long long)(q0 + 8 + q) * n) : 0.0;
         sl_read8<64>(tl + (uint32_t)q0, er, ecol + q0, v);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = __longlong_as_double(__double_as_longlong(v[q]) ^ flip);
+        if (__any_sync(0xFFFFFFFFu, add)) {  // (an FP64 add costs a warp 64 cycles)
+#pragma unroll
+            for (int q = 0; q < 8; ++q) v[q] = add ? v[q] + c[q] : v[q];
+        }
         if (mine) {
 #pragma unroll
             for (int q = 0; q < 8; ++q)
-                if (q0 + q < nc) dst[m + (long long)(q0 + q) * n] = base ? fma(sign, v[q], c[q]) : sign * v[q];
+                if (q0 + q < nc) dst[m + (long long)(q0 + q) * n] = v[q];
         }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) c[q] = cn[q];
     }
     tc_fence_before();
 }

@@ -1424,6 +1424,17 @@ __global__ void assemble_schur_kernel(const Tsrc *__restrict__ A_src, const T *_
 // ---------------------------------------------------------------------------
 constexpr int SOLVE_THREADS = 256;
 
+// Threads of a sweep's CTA.  256 finish a step soonest (the split sums of a
+// small block use them all) but hold an SM's registers with two CTAs; when
+// there are more partitions than two per SM, small blocks take fewer (one
+// right-hand side, n = 16, 1000 one-block partitions, forward: 12.2 us with
+// 256 threads, 4.1 us with 64; 30 partitions: 3.4 us against 3.6).
+inline int solve_threads(int n, int kc, long long partitions, int sms)
+{
+    if (partitions <= 2ll * sms) return SOLVE_THREADS;
+    return n * kc <= 16 ? 64 : n * kc <= 32 ? 128 : SOLVE_THREADS;
+}
+
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem)
 {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -1440,6 +1451,8 @@ __device__ __forceinline__ void cp_async4(void *smem, const void *gmem)
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem));
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
+// every group but the newest
+__device__ __forceinline__ void cp_async_wait_but1() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 // async copy of `count` contiguous elements (both ends aligned to 16 B when
@@ -1462,44 +1475,158 @@ __device__ __forceinline__ void async_copy(T *s, const T *__restrict__ g, int co
     }
 }
 
-// out(c, j) (+)= sign * sum_r M(r, c) v(r, j); M n x n (ld n), v/out n x kc (ld n).
-// A warp owns 4 output columns at a time; the four shuffle reductions are
-// interleaved so their latencies overlap.
-template <class T>
-__device__ __forceinline__ void cta_tmul(const T *sM, const T *v, T *out, int n, int kc, T sign, bool accumulate)
+// ---- transpose products of staged blocks ----
+// A vector of W consecutive elements of a column.
+template <class T, int W>
+struct VecN;
+template <>
+struct VecN<float, 4> {
+    using type = float4;
+};
+template <>
+struct VecN<float, 2> {
+    using type = float2;
+};
+template <>
+struct VecN<float, 1> {
+    using type = float;
+};
+template <>
+struct VecN<double, 2> {
+    using type = double2;
+};
+template <>
+struct VecN<double, 1> {
+    using type = double;
+};
+__device__ __forceinline__ void fma_vec(float &acc, const float2 &x, const float2 &y)
 {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int c0 = 4 * warp; c0 < n; c0 += 4 * nw) {
-        for (int j = 0; j < kc; ++j) {
-            T s[4] = {T(0), T(0), T(0), T(0)};
-            for (int r = lane; r < n; r += 32) {
-                const T vr = v[r + j * n];
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-                    if (c0 + q < n) s[q] = fma(sM[r + (c0 + q) * n], vr, s[q]);
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-                for (int q = 0; q < 4; ++q) s[q] += __shfl_xor_sync(0xffffffffu, s[q], o);
-            if (lane < 4 && c0 + lane < n) {
-                T val = s[0];
-#pragma unroll
-                for (int q = 1; q < 4; ++q)
-                    if (lane == q) val = s[q];
-                const int o = c0 + lane + j * n;
-                out[o] = accumulate ? out[o] + sign * val : sign * val;
+    acc = fmaf(x.x, y.x, acc);
+    acc = fmaf(x.y, y.y, acc);
+}
+__device__ __forceinline__ void fma_vec(float &acc, float x, float y) { acc = fmaf(x, y, acc); }
+__device__ __forceinline__ void fma_vec(double &acc, double x, double y) { acc = fma(x, y, acc); }
+
+// out(c, j) (+)= sign sum_r M(r, c) v(r, j) with M, v, out in shared memory
+// (leading dimension n), given as element offsets into it
+struct TmulOp {
+    int M, out;
+    bool minus, add;
+};
+
+// One or two such products with the same v (two to four right-hand sides at a
+// time).  A warp takes 8 CT columns x JT
+// right-hand sides: lane = column (lane % 8), share of the contraction (lane
+// / 8, every fourth chunk of W rows), the shares added by shuffles.  Each
+// lane starts its walk lane % 8 chunks in, so that the eight columns of an
+// access fall into distinct banks of the unpadded block.  tri: M upper
+// triangular, chunks wholly below the warp's columns are skipped.
+// What bounds it: in FP64 the FP64 pipe, whose instructions cost the same for
+// one lane as for 32, so a sum over 32 lanes by five shuffles costs as much
+// as 20 rows of FMAs (the form before this one: 14 us per 64-wide chain step,
+// k = 1; this one: 5 us); in FP32 with many columns the shared-memory reads,
+// 8 CT JT FMAs for CT + JT of them.
+template <class T, int W, int JT, int CT>
+__device__ __noinline__ void cta_tmul_t(const TmulOp a, const TmulOp b, int nops, int v0, int n, int kc, bool tri)
+{
+    using V = typename VecN<T, W>::type;
+    constexpr int JP = JT == 3 ? 4 : JT;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    T *sm = reinterpret_cast<T *>(smem_raw);
+    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    const int j8 = lane & 7, part = lane >> 3, nch = n / W;
+    const int G = (n + 8 * CT - 1) / (8 * CT), JG = (kc + JT - 1) / JT;
+    // this warp's tasks: every nw-th of (operation, right-hand-side group, column group)
+    int cg = threadIdx.x >> 5, jg = 0;
+    bool second = false;
+    for (;;) {
+        while (cg >= G) {
+            cg -= G;
+            if (++jg == JG) {
+                if (second || nops == 1) return;
+                jg = 0;
+                second = true;
             }
         }
+        const int j0 = JT * jg;
+        const T *M = sm + (second ? b.M : a.M);
+        T *out = sm + (second ? b.out : a.out);
+        const bool minus = second ? b.minus : a.minus, add = second ? b.add : a.add;
+        const int lim = tri ? min(nch, (8 * CT * (cg + 1) + W - 1) / W) : nch;
+        const T *mc[CT];
+#pragma unroll
+        for (int t = 0; t < CT; ++t) mc[t] = M + min(8 * (CT * cg + t) + j8, n - 1) * n;
+        const T *v[JT];  // (columns beyond the last repeat it: no branch between the reads)
+#pragma unroll
+        for (int j = 0; j < JT; ++j) v[j] = sm + v0 + min(j0 + j, kc - 1) * n;
+        T acc[JP * CT];  // (j, t), j padded to a power of two
+#pragma unroll
+        for (int i = 0; i < JP * CT; ++i) acc[i] = T(0);
+        int ch = part + j8;
+        while (ch >= lim) ch -= lim;
+#pragma unroll 2
+        for (int q = part; q < lim; q += 4) {
+            V m[CT];
+#pragma unroll
+            for (int t = 0; t < CT; ++t) m[t] = *reinterpret_cast<const V *>(mc[t] + ch * W);
+#pragma unroll
+            for (int j = 0; j < JT; ++j) {
+                const V y = *reinterpret_cast<const V *>(v[j] + ch * W);
+#pragma unroll
+                for (int t = 0; t < CT; ++t) fma_vec(acc[j * CT + t], m[t], y);
+            }
+            ch += 4;
+            if (ch >= lim) ch -= lim;
+        }
+        // the four shares' sums, each lane keeping a half, then a quarter of them
+        // (JP = 4: the lane's right-hand side is j0 + part)
+        constexpr int H = JP * CT / (JP >= 2 ? 2 : 1), Q = JP * CT / JP;
+        if constexpr (JP >= 2) {
+#pragma unroll
+            for (int i = 0; i < H; ++i) {
+                const bool up = (lane & 16) != 0;
+                const T send = up ? acc[i] : acc[i + H], keep = up ? acc[i + H] : acc[i];
+                acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < H; ++i) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], 16);
+        }
+        if constexpr (JP == 4) {
+#pragma unroll
+            for (int i = 0; i < Q; ++i) {
+                const bool up = (lane & 8) != 0;
+                const T send = up ? acc[i] : acc[i + Q], keep = up ? acc[i + Q] : acc[i];
+                acc[i] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < Q; ++i) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], 8);
+        }
+        const int j = JP == 4 ? part : JP == 2 ? part >> 1 : 0;
+        const bool writes = j < JT && j0 + j < kc && (JP == 4 || (part & (JP == 2 ? 1 : 3)) == 0);
+        if (writes) {
+#pragma unroll
+            for (int t = 0; t < CT; ++t) {
+                const int c = 8 * (CT * cg + t) + j8;
+                if (c < n) {
+                    T *o = out + c + (j0 + j) * n;
+                    const T x = minus ? -acc[t] : acc[t];
+                    *o = add ? *o + x : x;
+                }
+            }
+        }
+        cg += nw;
     }
 }
 
 // out(r, j) = base(r, j) + sign * (sum_c M1(r,c) v1(c,j) [+ sum_c M2(r,c) v2(c,j)])
-// (base may be null).  `red` holds max(blockDim, n*kc) elements.  Ends
-// without a barrier; callers sync before reading `out`.
+// (base may be null).  `red` holds max(blockDim, n*kc) elements.  tri: M1 is
+// upper triangular (no M2), columns below a half-warp's rows are skipped.
+// Ends without a barrier; callers sync before reading `out`.
 template <class T>
 __device__ __forceinline__ void cta_nmul(const T *M1, const T *v1, const T *M2, const T *v2, const T *base, T *out,
-                                         T sign, int n, int kc, T *red)
+                                         T sign, int n, int kc, T *red, bool tri)
 {
     const int no = n * kc;
     int parts = (int)blockDim.x / no;
@@ -1509,7 +1636,7 @@ __device__ __forceinline__ void cta_nmul(const T *M1, const T *v1, const T *M2, 
         const int j = o / n, r = o - j * n;
         const int c0 = (part * n) / parts, c1 = ((part + 1) * n) / parts;
         T s = T(0);
-        for (int c = c0; c < c1; ++c) s = fma(M1[r + c * n], v1[c + j * n], s);
+        for (int c = tri ? max(c0, r & ~15) : c0; c < c1; ++c) s = fma(M1[r + c * n], v1[c + j * n], s);
         if (M2)
             for (int c = c0; c < c1; ++c) s = fma(M2[r + c * n], v2[c + j * n], s);
         red[w] = s;
@@ -1649,55 +1776,18 @@ __device__ __forceinline__ void cta_nmul_g(const T *M1, const T *v1, const T *M2
     }
 }
 
-// Forms for a block staged in shared memory (leading dimension n, a multiple
+// Form for a block staged in shared memory (leading dimension n, a multiple
 // of the vector width W: 4 floats or 2 doubles, 16 bytes) and several
 // right-hand-side columns: every thread owns whole outputs, so no cross-lane
-// reduction is needed, and walks the contraction in 16-byte steps; the lanes
-// of a shared-memory wavefront start their walks at different offsets
-// (W (lane % 8) mod n) so that they hit distinct banks.
+// reduction is needed, and walks the contraction in 16-byte steps.
 //
-// out(c, j) (+)= sign * sum_r M(r, c) v(r, j): thread = (column c, the
-// right-hand sides jg, jg + tpc, ... with tpc = threads / n).
-template <class T>
-__device__ __forceinline__ void cta_tmul_s(const T *sM, const T *v, T *out, int n, int kc, T sign, bool accumulate)
-{
-    using VT = typename Vec<T>::type;
-    constexpr int W = Vec<T>::W;
-    const int tpc = (int)blockDim.x / n;
-    const int c = threadIdx.x % n, jg = threadIdx.x / n;
-    if (jg >= tpc) return;
-    const int rot = (W * (threadIdx.x & 7)) % n;
-    const T *mc = sM + (size_t)c * n;
-    for (int j0 = jg; j0 < kc; j0 += 4 * tpc) {
-        T acc[4] = {T(0), T(0), T(0), T(0)};
-        for (int r4 = 0; r4 < n; r4 += W) {
-            int r = r4 + rot;
-            if (r >= n) r -= n;
-            const VT m = *reinterpret_cast<const VT *>(mc + r);
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int j = j0 + tpc * q;
-                if (j < kc) fma_vec(acc[q], m, *reinterpret_cast<const VT *>(v + r + (size_t)j * n));
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int j = j0 + tpc * q;
-            if (j < kc) {
-                const int o = c + j * n;
-                out[o] = accumulate ? out[o] + sign * acc[q] : sign * acc[q];
-            }
-        }
-    }
-}
-
 // out(r, j) = base(r, j) + sign * (sum_c M1(r, c) v1(c, j) [+ sum_c M2(r, c)
 // v2(c, j)]) (base may be null, may be out): thread = (row r, right-hand sides
 // jg, jg + tpc, ...); M read along rows (lanes on consecutive rows), v as
 // 16-byte broadcasts.  No barrier.
 template <class T>
 __device__ __forceinline__ void cta_nmul_s(const T *M1, const T *v1, const T *M2, const T *v2, const T *base,
-                                           T *out, T sign, int n, int kc)
+                                           T *out, T sign, int n, int kc, bool tri)
 {
     using VT = typename Vec<T>::type;
     constexpr int W = Vec<T>::W;
@@ -1710,7 +1800,7 @@ __device__ __forceinline__ void cta_nmul_s(const T *M1, const T *v1, const T *M2
             const T *M = mi == 0 ? M1 : M2;
             const T *v = mi == 0 ? v1 : v2;
             if (!M) continue;
-            for (int c = 0; c < n; c += W) {
+            for (int c = tri ? r & ~15 : 0; c < n; c += W) {
                 T mrow[W];
 #pragma unroll
                 for (int w = 0; w < W; ++w) mrow[w] = M[r + (size_t)(c + w) * n];
@@ -1737,39 +1827,90 @@ __device__ __forceinline__ void cta_nmul_s(const T *M1, const T *v1, const T *M2
     }
 }
 
-// Staged blocks: the transpose product takes the register-blocked form when
-// there are several right-hand-side columns (every matrix element reused
-// across them; lanes run along rows, conflict-free on shared memory, no
-// scratch), the one-column form otherwise; the normal product keeps its
-// staged form.  Blocks read from global memory take the register-blocked
-// forms.
-template <bool STAGED, class T>
-__device__ __forceinline__ void tmul(const T *M, const T *v, T *out, int n, int kc, T sign, bool accumulate)
+// The same for one right-hand side, small enough to be inlined (the call and
+// its general bookkeeping cost 0.4 us of a 16-wide step's 1.6).
+template <class T, int W>
+__device__ __forceinline__ void cta_tmul_1(const TmulOp a, const TmulOp b, int nops, int v0, int n, bool tri)
 {
-    if constexpr (STAGED) {
-        if (kc > 1 && n % Vec<T>::W == 0 && n <= (int)blockDim.x) {
-            cta_tmul_s<T>(M, v, out, n, kc, sign, accumulate);
-            return;
+    using V = typename VecN<T, W>::type;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    T *sm = reinterpret_cast<T *>(smem_raw);
+    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    const int j8 = lane & 7, part = lane >> 3, nch = n / W, G = (n + 7) >> 3;
+    const T *v = sm + v0;
+    for (int u = threadIdx.x >> 5; u < nops * G; u += nw) {
+        const bool second = u >= G;
+        const int c8 = 8 * (second ? u - G : u), c = c8 + j8;
+        const int lim = tri ? min(nch, (c8 + 8 + W - 1) / W) : nch;
+        const T *m = sm + (second ? b.M : a.M) + min(c, n - 1) * n;
+        T acc = T(0);
+        int ch = part + j8;
+        while (ch >= lim) ch -= lim;
+#pragma unroll 4
+        for (int q = part; q < lim; q += 4) {
+            fma_vec(acc, *reinterpret_cast<const V *>(m + ch * W), *reinterpret_cast<const V *>(v + ch * W));
+            ch += 4;
+            if (ch >= lim) ch -= lim;
+        }
+        acc += __shfl_xor_sync(0xffffffffu, acc, 16);
+        acc += __shfl_xor_sync(0xffffffffu, acc, 8);
+        if (part == 0 && c < n) {
+            T *o = sm + (second ? b.out : a.out) + c;
+            const T x = (second ? b.minus : a.minus) ? -acc : acc;
+            *o = (second ? b.add : a.add) ? *o + x : x;
         }
     }
-    if (STAGED && kc == 1)
-        cta_tmul<T>(M, v, out, n, kc, sign, accumulate);
-    else
-        cta_tmul_g<T>(M, v, out, n, kc, sign, accumulate);
+}
+
+// Transpose products of blocks staged in shared memory: W = the widest vector
+// that every column starts on; with many right-hand sides in FP32 a warp takes
+// 2 or 4 column groups at once, as long as every warp still gets a task (each
+// matrix and vector read then feeds more FMAs).
+template <class T, int W>
+__device__ __forceinline__ void tmul_staged_w(const TmulOp a, const TmulOp b, int nops, int v, int n, int kc, bool tri)
+{
+    // right-hand sides per task: all of up to four, else three or four, whichever leaves fewer over
+    switch (kc <= 4 ? kc : (kc + (kc + 3) / 4 - 1) / ((kc + 3) / 4)) {
+    case 1: cta_tmul_1<T, W>(a, b, nops, v, n, tri); break;
+    case 2: cta_tmul_t<T, W, 2, 1>(a, b, nops, v, n, kc, tri); break;
+    case 3: cta_tmul_t<T, W, 3, 1>(a, b, nops, v, n, kc, tri); break;
+    default:
+        if constexpr (W == 4) {
+            const int tasks = nops * ((n + 7) / 8) * ((kc + 3) / 4), nw = (int)blockDim.x / 32;
+            if (tasks >= 4 * nw) cta_tmul_t<T, W, 4, 4>(a, b, nops, v, n, kc, tri);
+            else if (tasks >= 2 * nw) cta_tmul_t<T, W, 4, 2>(a, b, nops, v, n, kc, tri);
+            else cta_tmul_t<T, W, 4, 1>(a, b, nops, v, n, kc, tri);
+        } else {
+            cta_tmul_t<T, W, 4, 1>(a, b, nops, v, n, kc, tri);
+        }
+    }
+}
+template <class T>
+__device__ __forceinline__ void tmul_staged(const TmulOp a, const TmulOp b, int nops, int v, int n, int kc, bool tri)
+{
+    if constexpr (sizeof(T) == 8) {
+        if ((n & 1) == 0) tmul_staged_w<T, 2>(a, b, nops, v, n, kc, tri);
+        else tmul_staged_w<T, 1>(a, b, nops, v, n, kc, tri);
+    } else {
+        if ((n & 3) == 0) tmul_staged_w<T, 4>(a, b, nops, v, n, kc, tri);
+        else if ((n & 1) == 0) tmul_staged_w<T, 2>(a, b, nops, v, n, kc, tri);
+        else tmul_staged_w<T, 1>(a, b, nops, v, n, kc, tri);
+    }
 }
 
 // the staged multi-column form when there are more outputs than threads (else
-// the split contraction of cta_nmul keeps every thread busy)
+// the split contraction of cta_nmul keeps every thread busy); tri: M1 upper
+// triangular, no M2 (staged forms only: the others read every element anyway)
 template <bool STAGED, class T>
 __device__ __forceinline__ void nmul(const T *M1, const T *v1, const T *M2, const T *v2, const T *base, T *out,
-                                     T sign, int n, int kc, T *red)
+                                     T sign, int n, int kc, T *red, bool tri = false)
 {
     if constexpr (STAGED) {
         if (kc > 1 && n % Vec<T>::W == 0 && n * kc > (int)blockDim.x) {
-            cta_nmul_s<T>(M1, v1, M2, v2, base, out, sign, n, kc);
+            cta_nmul_s<T>(M1, v1, M2, v2, base, out, sign, n, kc, tri);
             return;
         }
-        cta_nmul<T>(M1, v1, M2, v2, base, out, sign, n, kc, red);
+        cta_nmul<T>(M1, v1, M2, v2, base, out, sign, n, kc, red, tri);
     } else {
         cta_nmul_g<T>(M1, v1, M2, v2, base, out, sign, n, kc, red);
     }
@@ -1881,55 +2022,65 @@ __device__ __forceinline__ void chain_fwd_body(const SolveArgs<T> &g, const long
     // step i uses V_i (slot 0), W_{i-1} (slot 1), Y_{i-1} (slot 2) and d_i in buffer
     // (i - first) & 1: the products with W_{i-1} (into this step's RHS) and Y_{i-1}
     // (into bL) both read y_{i-1}, so they share the step's first phase, and y_{i-1}
-    // is stored there too; the step's second phase is y_i = V_i^T r_i
-    if (STAGED) async_copy(buf, g.Af + first * (long long)nn, nn);
-    async_copy(srb, rhs_ptr<T>(g.d, first, n, g.k, g.j0), nkc);
-    cp_async_commit();
-    for (long long i = first; i <= last; ++i) {
+    // is stored there too; the step's second phase is y_i = V_i^T r_i.  Step last + 1
+    // of a partition has only the first phase: bR = W_last^T y_last, the last bL term
+    auto prefetch = [&](long long i) {  // what step i needs
+        const int cb = (int)((i - first) & 1);
+        T *to = buf + cb * 3 * nn;
+        if (i <= last) {
+            if (STAGED) async_copy(to, g.Af + i * (long long)nn, nn);
+            async_copy(srb + cb * nkc, rhs_ptr<T>(g.d, i, n, g.k, g.j0), nkc);
+        }
+        if (STAGED && i > first && (!seq || i <= last)) {
+            async_copy(to + nn, g.Bf + (i - 1) * (long long)nn, nn);
+            if (!seq) async_copy(to + 2 * nn, g.Y + (i - 1) * (long long)nn, nn);
+        }
+        cp_async_commit();
+        // blocks read straight from global memory are hinted into L2 instead
+        if (!STAGED && i > first && i <= last) {
+            prefetch_l2(g.Af + i * (long long)nn, (size_t)nn * sizeof(T));
+            prefetch_l2(g.Bf + (i - 1) * (long long)nn, (size_t)nn * sizeof(T));
+            if (!seq) prefetch_l2(g.Y + (i - 1) * (long long)nn, (size_t)nn * sizeof(T));
+        }
+    };
+    const long long end = seq ? last : last + 1;
+    prefetch(first);
+    prefetch(first + 1);  // both buffers are free: a short chain waits for memory once, not twice
+    for (long long i = first; i <= end; ++i) {
         const int cb = (int)((i - first) & 1);
         T *cur = buf + cb * 3 * nn;
-        T *nxt = buf + (cb ^ 1) * 3 * nn;
         T *sr = srb + cb * nkc;
-        cp_async_wait_all();
+        if (i == first)
+            cp_async_wait_but1();
+        else
+            cp_async_wait_all();
         __syncthreads();
-        // prefetch step i+1: V_{i+1} and d_{i+1}, and W_i, Y_i for its first phase
-        // (after the last step, W_last and Y_last for bR and the last bL term)
-        if (i < last) {
-            if (STAGED) async_copy(nxt, g.Af + (i + 1) * (long long)nn, nn);
-            async_copy(srb + (cb ^ 1) * nkc, rhs_ptr<T>(g.d, i + 1, n, g.k, g.j0), nkc);
-        }
-        if (STAGED && (!seq || i < last)) async_copy(nxt + nn, g.Bf + i * (long long)nn, nn);
-        if (STAGED && !seq) async_copy(nxt + 2 * nn, g.Y + i * (long long)nn, nn);
-        cp_async_commit();
-        // matrices of step i: staged in shared memory, or read straight from global
-        // memory (then the next step's are hinted into L2 while this one runs)
-        if (!STAGED && i < last) {
-            prefetch_l2(g.Af + (i + 1) * (long long)nn, (size_t)nn * sizeof(T));
-            prefetch_l2(g.Bf + i * (long long)nn, (size_t)nn * sizeof(T));
-            if (!seq) prefetch_l2(g.Y + i * (long long)nn, (size_t)nn * sizeof(T));
-        }
-        const T *mV = STAGED ? cur : g.Af + i * (long long)nn;
+        if (i > first && i < end) prefetch(i + 1);
+        // matrices of step i: staged in shared memory, or read straight from global memory
         if (i > first) {
-            const T *mW = STAGED ? cur + nn : g.Bf + (i - 1) * (long long)nn;
-            const T *mY = STAGED ? cur + 2 * nn : g.Y + (i - 1) * (long long)nn;
             store_rhs(g.d, sy, i - 1, n, g.k, g.j0, kc);
-            tmul<STAGED>(mW, sy, sr, n, kc, T(-1), true);
-            if (!seq) tmul<STAGED>(mY, sy, sbL, n, kc, T(1), true);
+            T *o1 = i <= last ? sr : sbR;
+            if constexpr (STAGED) {
+                const TmulOp a{(int)(cur + nn - buf), (int)(o1 - buf), i <= last, i <= last};
+                const TmulOp b{(int)(cur + 2 * nn - buf), (int)(sbL - buf), false, true};
+                tmul_staged<T>(a, b, seq ? 1 : 2, (int)(sy - buf), n, kc, false);
+            } else {
+                cta_tmul_g<T>(g.Bf + (i - 1) * (long long)nn, sy, o1, n, kc, i <= last ? T(-1) : T(1), i <= last);
+                if (!seq) cta_tmul_g<T>(g.Y + (i - 1) * (long long)nn, sy, sbL, n, kc, T(1), true);
+            }
             __syncthreads();
         }
-        tmul<STAGED>(mV, sr, sy, n, kc, T(1), false);
+        if (i <= last) {
+            if constexpr (STAGED) {
+                const TmulOp a{(int)(cur - buf), (int)(sy - buf), false, false};
+                tmul_staged<T>(a, a, 1, (int)(sr - buf), n, kc, true);
+            } else {
+                cta_tmul_g<T>(g.Af + i * (long long)nn, sr, sy, n, kc, T(1), false);
+            }
+        }
     }
     cp_async_wait_all();
-    __syncthreads();
-    store_rhs(g.d, sy, last, n, g.k, g.j0, kc);
     if (!seq) {
-        // bL += Y_last^T y_last, bR = W_last^T y_last (both prefetched in the last step)
-        const T *nb = buf + ((last + 1 - first) & 1) * 3 * nn;
-        const T *wl = STAGED ? nb + nn : g.Bf + last * (long long)nn;
-        const T *yl = STAGED ? nb + 2 * nn : g.Y + last * (long long)nn;
-        tmul<STAGED>(yl, sy, sbL, n, kc, T(1), true);
-        tmul<STAGED>(wl, sy, sbR, n, kc, T(1), false);
-        __syncthreads();
         T *bp = g.bvec + p * 2 * (long long)nkc;
         for (int e = threadIdx.x; e < nkc; e += blockDim.x) {
             bp[e] = sbL[e];
@@ -1937,6 +2088,8 @@ __device__ __forceinline__ void chain_fwd_body(const SolveArgs<T> &g, const long
         }
         return;
     }
+    __syncthreads();
+    store_rhs(g.d, sy, last, n, g.k, g.j0, kc);
     __syncthreads();  // every y_i is stored before the backward sweep reads them back
     // sequential level, backward: x_i = V_i (y_i - W_i x_{i+1}); step i uses
     // V_i (slot 0), W_i (slot 1) and y_i
@@ -1968,7 +2121,7 @@ __device__ __forceinline__ void chain_fwd_body(const SolveArgs<T> &g, const long
             nmul<STAGED, T>(mW, sx, nullptr, nullptr, sr, sr, T(-1), n, kc, red);
             __syncthreads();
         }
-        nmul<STAGED, T>(mV, sr, nullptr, nullptr, nullptr, sx, T(1), n, kc, red);
+        nmul<STAGED, T>(mV, sr, nullptr, nullptr, nullptr, sx, T(1), n, kc, red, true);
         __syncthreads();
         store_rhs(g.d, sx, i, n, g.k, g.j0, kc);
     }
@@ -2079,11 +2232,12 @@ __device__ __forceinline__ void chain_bwd_body(const SolveArgs<T> &g, const long
         const T *mY = STAGED ? cur + 2 * nn : g.Y + i * (long long)nn;
         nmul<STAGED, T>(mY, sxL, mW, sxn, sz, sz, T(-1), n, kc, red);
         __syncthreads();
-        nmul<STAGED, T>(mV, sz, nullptr, nullptr, nullptr, sxt, T(1), n, kc, red);
+        nmul<STAGED, T>(mV, sz, nullptr, nullptr, nullptr, sxt, T(1), n, kc, red, true);
         __syncthreads();
-        for (int e = threadIdx.x; e < n * kc; e += blockDim.x) sxn[e] = sxt[e];
         store_rhs(g.d, sxt, i, n, g.k, g.j0, kc);
-        __syncthreads();
+        T *x = sxn;  // x_i is the next step's x_{i+1}; the other buffer's readers have passed two barriers
+        sxn = sxt;
+        sxt = x;
     }
     cp_async_wait_all();
 }
@@ -3016,6 +3170,7 @@ __global__ void init_identity_kernel(T *A, long long first_blk, long long last_b
 
 }  // namespace bss
 
+#include "bss_chain16.cuh"
 #include "bss_chain64_tc.cuh"
 #include "bss_chain_f64_tc.cuh"
 #include "bss_chain128_f64_tc.cuh"

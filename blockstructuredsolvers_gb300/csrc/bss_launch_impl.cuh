@@ -33,7 +33,7 @@ static cudaError_t chain64_tc(const ChainFactorArgs<Tin, float> &a, cudaStream_t
 // FP64 chains of 17..64-wide blocks: products on the tensor cores by digits
 // (bss_chain_f64_tc.cuh).  Up to 16 a block's products are 128 full FP64
 // warp-instructions each (2.4K cycles an SM), about what cutting and putting
-// together the digits would take, and the FP64-pipe kernel stays.
+// together the digits would take, and the FP64-pipe kernel below serves.
 template <int NB>
 static cudaError_t chain_f64_tc(const ChainFactorArgs<double, double> &a, cudaStream_t s)
 {
@@ -42,6 +42,15 @@ static cudaError_t chain_f64_tc(const ChainFactorArgs<double, double> &a, cudaSt
     if (e != cudaSuccess) return e;
     cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     kern<<<a.seq ? 1u : (unsigned)a.Q, SL_THREADS, SlGeo<NB>::BYTES, s>>>(a);
+    count_launch();
+    return cudaGetLastError();
+}
+
+// blocks up to 16 wide (bss_chain16.cuh)
+template <class Tin, class T>
+static cudaError_t chain16(const ChainFactorArgs<Tin, T> &a, cudaStream_t s)
+{
+    chain16_kernel<Tin, T><<<a.seq ? 1u : (unsigned)a.Q, C16_THREADS, C16Geo<T>::BYTES, s>>>(a);
     count_launch();
     return cudaGetLastError();
 }
@@ -173,7 +182,7 @@ template <class Tin, class T>
 cudaError_t launch_chain_factor(const ChainFactorArgs<Tin, T> &a, cudaStream_t s)
 {
     switch (tile_for(a.n)) {
-    case 16: return chain_factor_nb<Tin, T, 16>(a, s);
+    case 16: return chain16<Tin, T>(a, s);
     case 32: return chain_factor_nb<Tin, T, 32>(a, s);
     case 64: return chain_factor_nb<Tin, T, 64>(a, s);
     case WIDE_CLASS: return wide_chain_factor<Tin, T>(a, s);
@@ -220,7 +229,7 @@ template <class Tin, class T>
 int chain_factor_ctas_per_sm(int n, int variant)
 {
     switch (tile_for(n)) {
-    case 16: return ctas_nb<Tin, T, 16>(variant);
+    case 16: return ctas_per_sm(chain16_kernel<Tin, T>, C16_THREADS, C16Geo<T>::BYTES);
     case 32: return ctas_nb<Tin, T, 32>(variant);
     case 64: return ctas_nb<Tin, T, 64>(variant);
     case WIDE_CLASS:
@@ -262,6 +271,16 @@ static bool stream_aligned(const SolveArgs<T> &a)
 }
 
 template <class T>
+static int sweep_threads(const SolveArgs<T> &a, bool staged)
+{
+    if (!staged || a.seq) return SOLVE_THREADS;
+    int dev = 0, sms = 1;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return solve_threads(a.n, a.kc, a.Q, sms);
+}
+
+template <class T>
 cudaError_t launch_chain_fwd(const SolveArgs<T> &a, cudaStream_t s)
 {
     if (!a.seq && solve_streamed<T>(a.n, a.kc) && stream_aligned(a)) {
@@ -279,7 +298,7 @@ cudaError_t launch_chain_fwd(const SolveArgs<T> &a, cudaStream_t s)
     cudaError_t e = set_solve_smem<T>((const void *)kern, smem);
     if (e != cudaSuccess) return e;
     const unsigned grid = a.seq ? 1u : (unsigned)a.Q;
-    kern<<<grid, SOLVE_THREADS, smem, s>>>(a);
+    kern<<<grid, sweep_threads<T>(a, staged), smem, s>>>(a);
     count_launch();
     return cudaGetLastError();
 }
@@ -301,7 +320,7 @@ cudaError_t launch_chain_bwd(const SolveArgs<T> &a, cudaStream_t s)
     auto kern = staged ? chain_bwd_kernel<T, Tsep, true> : chain_bwd_kernel<T, Tsep, false>;
     cudaError_t e = set_solve_smem<T>((const void *)kern, smem);
     if (e != cudaSuccess) return e;
-    kern<<<(unsigned)a.Q, SOLVE_THREADS, smem, s>>>(a);
+    kern<<<(unsigned)a.Q, sweep_threads<T>(a, staged), smem, s>>>(a);
     count_launch();
     return cudaGetLastError();
 }

@@ -681,13 +681,6 @@ SolveArgs<T> solve_args(bss_handle *h, int l, int j0, int kc)
     return make_solve_args<T>(h, l, j0, kc);
 }
 
-cudaError_t fwd_level(bss_handle *h, int l, int j0, int kc)
-{
-    const Level &L = h->levels[l];
-    if (L.t == F64) return launch_chain_fwd<double>(solve_args<double>(h, l, j0, kc), h->ls);
-    return launch_chain_fwd<float>(solve_args<float>(h, l, j0, kc), h->ls);
-}
-
 cudaError_t rhs_level(bss_handle *h, int l, int j0, int kc)
 {
     const Level &L = h->levels[l];
@@ -705,13 +698,49 @@ cudaError_t rhs_level(bss_handle *h, int l, int j0, int kc)
     return cudaErrorInvalidValue;
 }
 
+// forward sweep of level l; below the finest level it forms its RHS from the
+// level above's results itself, unless the streamed kernel serves it or the
+// levels' types differ
+template <class T>
+cudaError_t fwd_level_t(bss_handle *h, int l, int j0, int kc)
+{
+    SolveArgs<T> a = solve_args<T>(h, l, j0, kc);
+    if (l > 0) {
+        const Level &F = h->levels[l - 1];
+        if (F.t == h->levels[l].t && !chain_fwd_streams<T>(a)) {
+            a.fine_d = (const T *)F.d;
+            a.fine_b = (const T *)F.bvec;
+            a.fine_N = F.N;
+            a.fine_Q = F.Q;
+            a.chained = 1;
+        } else {
+            const cudaError_t e = rhs_level(h, l - 1, j0, kc);
+            if (e != cudaSuccess) return e;
+        }
+    }
+    return launch_chain_fwd<T>(a, h->ls);
+}
+
+cudaError_t fwd_level(bss_handle *h, int l, int j0, int kc)
+{
+    return h->levels[l].t == F64 ? fwd_level_t<double>(h, l, j0, kc) : fwd_level_t<float>(h, l, j0, kc);
+}
+
+template <class T, class Tsep>
+cudaError_t bwd_level_t(bss_handle *h, int l, int j0, int kc)
+{
+    SolveArgs<T> a = solve_args<T>(h, l, j0, kc);
+    a.chained = 1;  // behind the next level's sweep
+    return launch_chain_bwd<T, Tsep>(a, h->ls);
+}
+
 cudaError_t bwd_level(bss_handle *h, int l, int j0, int kc)
 {
     const Level &L = h->levels[l];
     const Level &X = h->levels[l + 1];
-    if (L.t == F64 && X.t == F64) return launch_chain_bwd<double, double>(solve_args<double>(h, l, j0, kc), h->ls);
-    if (L.t == F32 && X.t == F32) return launch_chain_bwd<float, float>(solve_args<float>(h, l, j0, kc), h->ls);
-    if (L.t == F32 && X.t == F64) return launch_chain_bwd<float, double>(solve_args<float>(h, l, j0, kc), h->ls);
+    if (L.t == F64 && X.t == F64) return bwd_level_t<double, double>(h, l, j0, kc);
+    if (L.t == F32 && X.t == F32) return bwd_level_t<float, float>(h, l, j0, kc);
+    if (L.t == F32 && X.t == F64) return bwd_level_t<float, double>(h, l, j0, kc);
     return cudaErrorInvalidValue;
 }
 
@@ -721,11 +750,7 @@ int chain_solve(bss_handle *h)
     const int nlev = (int)h->levels.size();
     for (int j0 = 0; j0 < h->k; j0 += h->kc_max) {
         const int kc = (int)std::min<long long>(h->kc_max, h->k - j0);
-        for (int l = 0; l + 1 < nlev; ++l) {
-            BSS_CUDA(fwd_level(h, l, j0, kc));
-            BSS_CUDA(rhs_level(h, l, j0, kc));
-        }
-        BSS_CUDA(fwd_level(h, nlev - 1, j0, kc));  // sequential coarsest: fwd + bwd
+        for (int l = 0; l < nlev; ++l) BSS_CUDA(fwd_level(h, l, j0, kc));  // sequential coarsest: fwd + bwd
         for (int l = nlev - 2; l >= 0; --l) BSS_CUDA(bwd_level(h, l, j0, kc));
     }
     return BSS_OK;

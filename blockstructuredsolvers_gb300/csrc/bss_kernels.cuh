@@ -1898,6 +1898,33 @@ __device__ __forceinline__ void tmul_staged(const TmulOp a, const TmulOp b, int 
     }
 }
 
+// One right-hand side, staged blocks: a warp takes 8 rows, lane = row (lane %
+// 8), share of the columns (lane / 8, every fourth), the shares added by two
+// shuffles: no scratch and no barrier inside, where cta_nmul has one.  For
+// FP64, and FP32 up to n = 32: beyond, FP32's four shares of a column stride
+// that is a multiple of 32 words meet in the same banks, which costs more.
+template <class T>
+__device__ __forceinline__ void cta_nmul_1(const T *M1, const T *v1, const T *M2, const T *v2, const T *base, T *out,
+                                           T sign, int n, bool tri)
+{
+    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5, part = lane >> 3;
+    for (int r0 = 8 * (threadIdx.x >> 5); r0 < n; r0 += 8 * nw) {
+        const int r = r0 + (lane & 7), rr = min(r, n - 1);
+        T s = T(0);
+#pragma unroll 4
+        for (int c = (tri ? r0 : 0) + part; c < n; c += 4) s = fma(M1[rr + c * n], v1[c], s);
+        if (M2) {
+            T s2 = T(0);
+#pragma unroll 4
+            for (int c = part; c < n; c += 4) s2 = fma(M2[rr + c * n], v2[c], s2);
+            s += s2;
+        }
+        s += __shfl_xor_sync(0xffffffffu, s, 16);
+        s += __shfl_xor_sync(0xffffffffu, s, 8);
+        if (part == 0 && r < n) out[r] = (base ? base[r] : T(0)) + sign * s;
+    }
+}
+
 // the staged multi-column form when there are more outputs than threads (else
 // the split contraction of cta_nmul keeps every thread busy); tri: M1 upper
 // triangular, no M2 (staged forms only: the others read every element anyway)
@@ -1906,6 +1933,10 @@ __device__ __forceinline__ void nmul(const T *M1, const T *v1, const T *M2, cons
                                      T sign, int n, int kc, T *red, bool tri = false)
 {
     if constexpr (STAGED) {
+        if (kc == 1 && (sizeof(T) == 8 || n <= 32)) {
+            cta_nmul_1<T>(M1, v1, M2, v2, base, out, sign, n, tri);
+            return;
+        }
         if (kc > 1 && n % Vec<T>::W == 0 && n * kc > (int)blockDim.x) {
             cta_nmul_s<T>(M1, v1, M2, v2, base, out, sign, n, kc, tri);
             return;
@@ -1942,7 +1973,20 @@ struct SolveArgs {
     int kc;        // columns in this pass
     int seq;
     DevStatus *st; // a bounded wait of the streamed sweeps records its expiry here
+    // forward sweep of a coarser level straight from the finer level's results
+    // (its RHS, Q x [bL | bR], sizes): the level's own RHS is formed as it is read
+    const T *fine_d = nullptr, *fine_b = nullptr;
+    long long fine_N = 0, fine_Q = 0;
+    int chained = 0;  // launched behind another sweep of the same solve (programmatic dependence)
 };
+
+// Programmatic dependent launch: a sweep lets the next one's CTAs start as
+// soon as all its own have (they load factors, which no sweep writes), and
+// waits itself for the one before it, completed and visible, ahead of its
+// first access to anything a sweep writes.  Without the launch attribute both
+// are no-ops.
+__device__ __forceinline__ void pdl_release_next() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void pdl_wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // shared memory: 2 buffers x 3 blocks (staged form only) + 6 vectors +
 // reduction scratch.  Blocks too large to stage (n > 64 in FP64, n > 90 in
@@ -1992,9 +2036,43 @@ __device__ __forceinline__ void store_rhs(Tg *__restrict__ g, const T *s, long l
     for (int e = threadIdx.x; e < n * kc; e += blockDim.x) b[e] = (Tg)s[e];
 }
 
+// x - l - r rounded once: FP32 by error-free differences (Knuth's TwoSum),
+// whose FP32 instructions are far cheaper here than three conversions to FP64
+__device__ __forceinline__ double minus_both(double x, double l, double r) { return x - l - r; }
+__device__ __forceinline__ float minus_both(float x, float l, float r)
+{
+    const float s = __fsub_rn(x, l), sb = __fsub_rn(s, x);
+    const float es = __fsub_rn(__fsub_rn(x, __fsub_rn(s, sb)), __fadd_rn(l, sb));
+    const float t = __fsub_rn(s, r), tb = __fsub_rn(t, s);
+    const float et = __fsub_rn(__fsub_rn(s, __fsub_rn(t, tb)), __fadd_rn(r, tb));
+    const float y = __fadd_rn(t, __fadd_rn(es, et));
+    return isfinite(y) ? y : t;  // (an infinity makes the error terms NaN)
+}
+
+// block s of a coarser level's RHS, from the finer level's: d'_s = d_{sep s} -
+// bL(s) - bR(s-1) (as assemble_rhs_kernel).  Made ahead of the wait for the
+// finer level's sweep: the 64-bit division takes longer than a small product.
+template <class T>
+struct SepSource {
+    const T *d, *l, *r;  // null where block s has no such term
+    __device__ __forceinline__ SepSource(const SolveArgs<T> &g, long long s)
+    {
+        const long long per = (long long)g.n * g.kc, blk = (s * (g.fine_N - 1)) / g.fine_Q;
+        d = g.fine_d + blk * (long long)g.n * g.k + (long long)g.j0 * g.n;
+        l = s < g.fine_Q ? g.fine_b + s * 2 * per : nullptr;
+        r = s > 0 ? g.fine_b + (s - 1) * 2 * per + per : nullptr;
+    }
+    __device__ __forceinline__ void copy(T *to, int count) const
+    {
+        for (int e = threadIdx.x; e < count; e += blockDim.x)
+            to[e] = minus_both(d[e], l ? l[e] : T(0), r ? r[e] : T(0));
+    }
+};
+
 // forward sweep of one partition; for the sequential (coarsest) level the
 // whole chain followed by its backward sweep.
-template <class T, bool STAGED>
+// FUSED: the level's RHS is formed from the finer level's (g.fine_*).
+template <class T, bool STAGED, bool FUSED>
 __device__ __forceinline__ void chain_fwd_body(const SolveArgs<T> &g, const long long p)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -2024,18 +2102,14 @@ __device__ __forceinline__ void chain_fwd_body(const SolveArgs<T> &g, const long
     // (into bL) both read y_{i-1}, so they share the step's first phase, and y_{i-1}
     // is stored there too; the step's second phase is y_i = V_i^T r_i.  Step last + 1
     // of a partition has only the first phase: bR = W_last^T y_last, the last bL term
-    auto prefetch = [&](long long i) {  // what step i needs
+    auto fetch_blocks = [&](long long i) {
         const int cb = (int)((i - first) & 1);
         T *to = buf + cb * 3 * nn;
-        if (i <= last) {
-            if (STAGED) async_copy(to, g.Af + i * (long long)nn, nn);
-            async_copy(srb + cb * nkc, rhs_ptr<T>(g.d, i, n, g.k, g.j0), nkc);
-        }
+        if (STAGED && i <= last) async_copy(to, g.Af + i * (long long)nn, nn);
         if (STAGED && i > first && (!seq || i <= last)) {
             async_copy(to + nn, g.Bf + (i - 1) * (long long)nn, nn);
             if (!seq) async_copy(to + 2 * nn, g.Y + (i - 1) * (long long)nn, nn);
         }
-        cp_async_commit();
         // blocks read straight from global memory are hinted into L2 instead
         if (!STAGED && i > first && i <= last) {
             prefetch_l2(g.Af + i * (long long)nn, (size_t)nn * sizeof(T));
@@ -2043,9 +2117,35 @@ __device__ __forceinline__ void chain_fwd_body(const SolveArgs<T> &g, const long
             if (!seq) prefetch_l2(g.Y + (i - 1) * (long long)nn, (size_t)nn * sizeof(T));
         }
     };
+    auto fetch_rhs = [&](long long i) {
+        if (i > last) return;
+        T *to = srb + ((i - first) & 1) * nkc;
+        if constexpr (FUSED)
+            SepSource<T>(g, i).copy(to, nkc);
+        else
+            async_copy(to, rhs_ptr<T>(g.d, i, n, g.k, g.j0), nkc);
+    };
     const long long end = seq ? last : last + 1;
-    prefetch(first);
-    prefetch(first + 1);  // both buffers are free: a short chain waits for memory once, not twice
+    // a short chain waits for memory once: both buffers are free, and the factors
+    // do not depend on the sweep before this one
+    pdl_release_next();
+    fetch_blocks(first);
+    if constexpr (FUSED) {
+        cp_async_commit();
+        fetch_blocks(first + 1);
+        cp_async_commit();
+        const SepSource<T> s0(g, first), s1(g, first < last ? first + 1 : first);
+        pdl_wait_previous();
+        s0.copy(srb, nkc);
+        if (first < last) s1.copy(srb + nkc, nkc);
+    } else {
+        pdl_wait_previous();
+        fetch_rhs(first);
+        cp_async_commit();
+        fetch_blocks(first + 1);
+        fetch_rhs(first + 1);
+        cp_async_commit();
+    }
     for (long long i = first; i <= end; ++i) {
         const int cb = (int)((i - first) & 1);
         T *cur = buf + cb * 3 * nn;
@@ -2055,7 +2155,11 @@ __device__ __forceinline__ void chain_fwd_body(const SolveArgs<T> &g, const long
         else
             cp_async_wait_all();
         __syncthreads();
-        if (i > first && i < end) prefetch(i + 1);
+        if (i > first && i < end) {
+            fetch_blocks(i + 1);
+            fetch_rhs(i + 1);
+            cp_async_commit();
+        }
         // matrices of step i: staged in shared memory, or read straight from global memory
         if (i > first) {
             store_rhs(g.d, sy, i - 1, n, g.k, g.j0, kc);
@@ -2081,6 +2185,10 @@ __device__ __forceinline__ void chain_fwd_body(const SolveArgs<T> &g, const long
     }
     cp_async_wait_all();
     if (!seq) {
+        if constexpr (FUSED) {  // this level's separators, read by the next one
+            SepSource<T>(g, first - 1).copy(const_cast<T *>(rhs_ptr<T>(g.d, first - 1, n, g.k, g.j0)), nkc);
+            if (p == g.Q - 1) SepSource<T>(g, last + 1).copy(const_cast<T *>(rhs_ptr<T>(g.d, last + 1, n, g.k, g.j0)), nkc);
+        }
         T *bp = g.bvec + p * 2 * (long long)nkc;
         for (int e = threadIdx.x; e < nkc; e += blockDim.x) {
             bp[e] = sbL[e];
@@ -2128,10 +2236,10 @@ __device__ __forceinline__ void chain_fwd_body(const SolveArgs<T> &g, const long
     cp_async_wait_all();
 }
 
-template <class T, bool STAGED>
+template <class T, bool STAGED, bool FUSED>
 __global__ void __launch_bounds__(SOLVE_THREADS, 2) chain_fwd_kernel(SolveArgs<T> g)
 {
-    chain_fwd_body<T, STAGED>(g, blockIdx.x);
+    chain_fwd_body<T, STAGED, FUSED>(g, blockIdx.x);
 }
 
 template <class T, bool STAGED>
@@ -2148,7 +2256,7 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 2)
         if (it >= nitems) break;
         const WorkItem w = items[it];
         const SolveArgs<T> g = descs[w.desc];
-        chain_fwd_body<T, STAGED>(g, w.p);
+        chain_fwd_body<T, STAGED, false>(g, w.p);
         __syncthreads();
     }
 }
@@ -2194,11 +2302,13 @@ __device__ __forceinline__ void chain_bwd_body(const SolveArgs<T> &g, const long
     const long long sR = ((p + 1) * (g.N - 1)) / g.Q;
     const long long first = sL + 1, last = sR - 1;
     const Tsep *xs = reinterpret_cast<const Tsep *>(g.xsep);
+    pdl_release_next();
     if (STAGED) {
         async_copy(buf, g.Af + last * (long long)nn, nn);
         async_copy(buf + nn, g.Bf + last * (long long)nn, nn);
         async_copy(buf + 2 * nn, g.Y + last * (long long)nn, nn);
     }
+    pdl_wait_previous();
     async_copy(szb, rhs_ptr<T>(g.d, last, n, g.k, g.j0), nkc);
     cp_async_commit();
     load_rhs(sxL, xs, p, n, g.k, g.j0, kc);

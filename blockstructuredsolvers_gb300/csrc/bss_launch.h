@@ -34,6 +34,10 @@ cudaError_t launch_assemble_schur(const Tsrc *A_src, const T *C, Tdst *A_next, T
 
 template <class T>
 cudaError_t launch_chain_fwd(const SolveArgs<T> &a, cudaStream_t s);
+// whether launch_chain_fwd takes the streamed kernel, which reads the level's
+// RHS from memory (the others can form it from the finer level's, fine_d)
+template <class T>
+bool chain_fwd_streams(const SolveArgs<T> &a);
 template <class T, class Tsep>
 cudaError_t launch_chain_bwd(const SolveArgs<T> &a, cudaStream_t s);
 template <class T, class Tn>

@@ -270,6 +270,23 @@ static bool stream_aligned(const SolveArgs<T> &a)
     return (m & 15u) == 0 && ((size_t)a.n * sizeof(T)) % 16 == 0;
 }
 
+// launch with programmatic dependence on the kernel before it in the stream
+template <class... P, class... A>
+static cudaError_t launch_chained(void (*kern)(P...), unsigned grid, int threads, size_t smem, cudaStream_t s, A... args)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
 template <class T>
 static int sweep_threads(const SolveArgs<T> &a, bool staged)
 {
@@ -281,9 +298,15 @@ static int sweep_threads(const SolveArgs<T> &a, bool staged)
 }
 
 template <class T>
+bool chain_fwd_streams(const SolveArgs<T> &a)
+{
+    return !a.seq && solve_streamed<T>(a.n, a.kc) && stream_aligned(a);
+}
+
+template <class T>
 cudaError_t launch_chain_fwd(const SolveArgs<T> &a, cudaStream_t s)
 {
-    if (!a.seq && solve_streamed<T>(a.n, a.kc) && stream_aligned(a)) {
+    if (chain_fwd_streams(a)) {
         const size_t smem = stream_smem_bytes<T>(a.n, a.kc);
         auto kern = chain_fwd_stream_kernel<T>;
         cudaError_t e = set_solve_smem<T>((const void *)kern, smem);
@@ -294,13 +317,15 @@ cudaError_t launch_chain_fwd(const SolveArgs<T> &a, cudaStream_t s)
     }
     const bool staged = solve_staged<T>(a.n, a.kc);
     const size_t smem = solve_smem_bytes<T>(a.n, a.kc, staged);
-    auto kern = staged ? chain_fwd_kernel<T, true> : chain_fwd_kernel<T, false>;
+    auto kern = a.fine_d ? (staged ? chain_fwd_kernel<T, true, true> : chain_fwd_kernel<T, false, true>)
+                         : (staged ? chain_fwd_kernel<T, true, false> : chain_fwd_kernel<T, false, false>);
     cudaError_t e = set_solve_smem<T>((const void *)kern, smem);
     if (e != cudaSuccess) return e;
     const unsigned grid = a.seq ? 1u : (unsigned)a.Q;
-    kern<<<grid, sweep_threads<T>(a, staged), smem, s>>>(a);
+    if (a.chained) e = launch_chained(kern, grid, sweep_threads<T>(a, staged), smem, s, a);
+    else kern<<<grid, sweep_threads<T>(a, staged), smem, s>>>(a);
     count_launch();
-    return cudaGetLastError();
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 template <class T, class Tsep>
@@ -320,9 +345,10 @@ cudaError_t launch_chain_bwd(const SolveArgs<T> &a, cudaStream_t s)
     auto kern = staged ? chain_bwd_kernel<T, Tsep, true> : chain_bwd_kernel<T, Tsep, false>;
     cudaError_t e = set_solve_smem<T>((const void *)kern, smem);
     if (e != cudaSuccess) return e;
-    kern<<<(unsigned)a.Q, sweep_threads<T>(a, staged), smem, s>>>(a);
+    if (a.chained) e = launch_chained(kern, (unsigned)a.Q, sweep_threads<T>(a, staged), smem, s, a);
+    else kern<<<(unsigned)a.Q, sweep_threads<T>(a, staged), smem, s>>>(a);
     count_launch();
-    return cudaGetLastError();
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 template <class T, class Tn>

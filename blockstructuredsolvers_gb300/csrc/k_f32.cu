@@ -10,6 +10,7 @@ template cudaError_t launch_assemble_schur<float, float, float>(const float *, c
 template cudaError_t launch_assemble_schur<float, float, double>(const float *, const float *, double *, double *,
                                                                  long long, long long, int, cudaStream_t);
 template cudaError_t launch_chain_fwd<float>(const SolveArgs<float> &, cudaStream_t);
+template bool chain_fwd_streams<float>(const SolveArgs<float> &);
 template cudaError_t launch_chain_bwd<float, float>(const SolveArgs<float> &, cudaStream_t);
 template cudaError_t launch_chain_bwd<float, double>(const SolveArgs<float> &, cudaStream_t);
 template cudaError_t launch_assemble_rhs<float, float>(const float *, const float *, float *, long long, long long,

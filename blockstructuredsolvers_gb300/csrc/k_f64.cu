@@ -8,6 +8,7 @@ template cudaError_t launch_assemble_schur<double, double, double>(const double 
                                                                    double *, long long, long long, int,
                                                                    cudaStream_t);
 template cudaError_t launch_chain_fwd<double>(const SolveArgs<double> &, cudaStream_t);
+template bool chain_fwd_streams<double>(const SolveArgs<double> &);
 template cudaError_t launch_chain_bwd<double, double>(const SolveArgs<double> &, cudaStream_t);
 template cudaError_t launch_assemble_rhs<double, double>(const double *, const double *, double *, long long,
                                                          long long, int, int, int, int, cudaStream_t);

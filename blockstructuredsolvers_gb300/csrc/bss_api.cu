@@ -550,16 +550,9 @@ cudaError_t factor_any(bss_handle *h, int l)
 
 static int factorize_upto(bss_handle *h, int upto)
 {
-    BSS_CUDA(cudaMemsetAsync(&h->st->bad_key, 0xFF, sizeof(unsigned long long), h->ls));
-    BSS_CUDA(cudaMemsetAsync(&h->st->tc_timeout, 0, sizeof(int), h->ls));
     const bool mixed = h->opt.precision == BSS_PRECISION_MIXED;
-    if (mixed) {
-        // ||T||_inf is folded into the first residual after this factorization
-        BSS_CUDA(cudaMemsetAsync(&h->st->anorm, 0, sizeof(unsigned long long), h->ls));
-        BSS_CUDA(cudaMemsetAsync(&h->st->need_anorm, 0, sizeof(int), h->ls));
-        BSS_CUDA(cudaMemsetAsync(&h->st->need_anorm, 1, 1, h->ls));
-        h->need_anorm = true;
-    }
+    BSS_CUDA(launch_factor_status(h->st, mixed ? 1 : 0, h->ls));
+    if (mixed) h->need_anorm = true;  // ||T||_inf is folded into the first residual after this factorization
     const int nlev = (int)h->levels.size();
     for (int l = 0; l < nlev && l < upto; ++l) {
         BSS_CUDA(factor_any(h, l));
@@ -771,10 +764,8 @@ int residual_check(bss_handle *h)
 {
     const double *d64 = (const double *)h->d;
     DevStatus *st = h->st;
-    BSS_CUDA(cudaMemsetAsync(&st->rnorm, 0, 2 * sizeof(unsigned long long), h->ls));
-    const int wn = h->need_anorm ? 1 : 0;
+    const int wn = h->need_anorm ? 1 : 0;  // (the norms are clear: rhs_begin, then each relres)
     h->need_anorm = false;
-    if (wn) BSS_CUDA(cudaMemsetAsync(&st->need_anorm, 0, sizeof(int), h->ls));
     if (h->levels[0].t == F32)
         BSS_CUDA((launch_residual_df<float>((const double *)h->A, (const double *)h->B, h->x64, d64,
                                             (float *)h->c0, h->N, (int)h->n, (int)h->k, wn, st, h->ls)));
@@ -794,12 +785,10 @@ int bss::mixed_begin(bss_handle *h)
 {
     const long long cnt = h->N * h->n * h->k;
     const double *d64 = (const double *)h->d;
-    BSS_CUDA(cudaMemsetAsync(&h->st->dnorm, 0, sizeof(unsigned long long), h->ls));
-    BSS_CUDA(launch_absmax<double>(d64, cnt, &h->st->dnorm, h->ls));
     if (h->levels[0].t == F32)
-        BSS_CUDA((launch_convert<double, float>((float *)h->c0, d64, cnt, h->ls)));
+        BSS_CUDA(launch_rhs_begin<float>((float *)h->c0, d64, cnt, h->st, h->ls));
     else
-        BSS_CUDA((launch_convert<double, double>((double *)h->c0, d64, cnt, h->ls)));
+        BSS_CUDA(launch_rhs_begin<double>((double *)h->c0, d64, cnt, h->st, h->ls));
     int rc = chain_solve(h);
     if (rc) return rc;
     if (h->levels[0].t == F32)
@@ -872,14 +861,10 @@ int capture_mixed_solve(bss_handle *h)
     const bool c_is_f32 = h->levels[0].t == F32;
     DevStatus *st = h->st;
     const long long k0 = launch_count();
-    BSS_CUDA(cudaMemsetAsync(&st->dnorm, 0, sizeof(unsigned long long), h->ls));
-    BSS_CUDA(cudaMemsetAsync(&st->iters, 0, sizeof(int), h->ls));
-    BSS_CUDA(cudaMemsetAsync(&st->done, 0, sizeof(int), h->ls));
-    BSS_CUDA(launch_absmax<double>(d64, cnt, &st->dnorm, h->ls));
     if (c_is_f32)
-        BSS_CUDA((launch_convert<double, float>((float *)h->c0, d64, cnt, h->ls)));
+        BSS_CUDA(launch_rhs_begin<float>((float *)h->c0, d64, cnt, st, h->ls));
     else
-        BSS_CUDA((launch_convert<double, double>((double *)h->c0, d64, cnt, h->ls)));
+        BSS_CUDA(launch_rhs_begin<double>((double *)h->c0, d64, cnt, st, h->ls));
     int rc = chain_solve(h);
     if (rc) return rc;
     if (c_is_f32)
@@ -909,7 +894,6 @@ int capture_mixed_solve(bss_handle *h)
     // loop body: residual + decision, then the conditional correction
     h->ls = h->cap_stream2;
     BSS_CUDA(cudaStreamBeginCaptureToGraph(h->cap_stream2, wbody, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
-    BSS_CUDA(cudaMemsetAsync(&st->rnorm, 0, 2 * sizeof(unsigned long long), h->ls));
     if (c_is_f32)
         BSS_CUDA((launch_residual_df<float>((const double *)h->A, (const double *)h->B, h->x64, d64,
                                             (float *)h->c0, h->N, (int)h->n, (int)h->k, -1, st, h->ls)));

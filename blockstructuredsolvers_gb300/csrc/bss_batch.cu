@@ -173,6 +173,42 @@ cudaError_t queue_factor_wide(const ChainFactorArgs<Tin, T> *descs, const WorkIt
     return cudaGetLastError();
 }
 
+// the tensor-core chain kernels of the single-system path, for partitioned
+// levels with FP32 factors (33..64 and 65..128 wide)
+template <class Tin>
+cudaError_t queue_factor64_tc(const ChainFactorArgs<Tin, float> *descs, const WorkItem *items, int nitems, int *head,
+                              int sms, cudaStream_t s)
+{
+    const size_t smem = chain64_tc_smem();
+    auto kern = chain64_tc_kernel<Tin, true>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    const int grid = std::max(1, std::min(nitems, sms * ctas_per_sm(kern, C64_THREADS, smem)));
+    e = cudaMemsetAsync(head, 0, sizeof(int), s);
+    if (e != cudaSuccess) return e;
+    kern<<<grid, C64_THREADS, smem, s>>>(ChainFactorArgs<Tin, float>{}, descs, items, nitems, head);
+    count_launch();
+    return cudaGetLastError();
+}
+
+template <class Tin>
+cudaError_t queue_factor128_tc(const ChainFactorArgs<Tin, float> *descs, const CUtensorMap *maps, bool tma,
+                               const WorkItem *items, int nitems, int *head, int sms, cudaStream_t s)
+{
+    const size_t smem = chain128_tc_smem();
+    auto kern = chain128_tc_kernel<Tin, true>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+    e = cudaMemsetAsync(head, 0, sizeof(int), s);
+    if (e != cudaSuccess) return e;
+    kern<<<std::min(nitems, sms), C128_THREADS, smem, s>>>(ChainFactorArgs<Tin, float>{}, CUtensorMap{}, tma ? 1 : 0,
+                                                          descs, maps, items, nitems, head);
+    count_launch();
+    return cudaGetLastError();
+}
+
 template <class Tin, class T>
 cudaError_t queue_factor(int nb, const ChainFactorArgs<Tin, T> *descs, const WorkItem *items, int nitems, int *head,
                          int sms, cudaStream_t s)
@@ -187,11 +223,29 @@ cudaError_t queue_factor(int nb, const ChainFactorArgs<Tin, T> *descs, const Wor
     }
 }
 
+// how a launch of sweeps reads the blocks: straight from global memory, whole
+// steps staged, or streamed through a ring (wide blocks of partitioned levels)
+enum SweepForm { SWEEP_DIRECT, SWEEP_STAGED, SWEEP_STREAMED };
+
 template <class T>
-cudaError_t queue_fwd(const SolveArgs<T> *descs, const WorkItem *items, int nitems, int *head, size_t smem, int sms,
-                      bool staged, cudaStream_t s)
+SweepForm sweep_form(const bss_handle *h, bool coarsest_fwd)
 {
-    auto kern = staged ? chain_fwd_queue_kernel<T, true> : chain_fwd_queue_kernel<T, false>;
+    const int n = (int)h->n, k = (int)h->k;
+    if (solve_staged<T>(n, k)) return SWEEP_STAGED;
+    return !coarsest_fwd && solve_streamed<T>(n, k) ? SWEEP_STREAMED : SWEEP_DIRECT;
+}
+template <class T>
+size_t sweep_smem(const bss_handle *h, SweepForm f)
+{
+    const int n = (int)h->n, k = (int)h->k;
+    return f == SWEEP_STREAMED ? stream_smem_bytes<T>(n, k) : solve_smem_bytes<T>(n, k, f == SWEEP_STAGED);
+}
+const char *sweep_name(SweepForm f) { return f == SWEEP_STAGED ? " staged" : f == SWEEP_STREAMED ? " streamed" : " direct"; }
+
+template <class T>
+cudaError_t queue_sweep(void (*kern)(const SolveArgs<T> *, const WorkItem *, int, int *), const SolveArgs<T> *descs,
+                        const WorkItem *items, int nitems, int *head, size_t smem, int sms, cudaStream_t s)
+{
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     int per = 1;
@@ -204,21 +258,22 @@ cudaError_t queue_fwd(const SolveArgs<T> *descs, const WorkItem *items, int nite
     return cudaGetLastError();
 }
 
+template <class T>
+cudaError_t queue_fwd(const SolveArgs<T> *descs, const WorkItem *items, int nitems, int *head, size_t smem, int sms,
+                      SweepForm f, cudaStream_t s)
+{
+    auto kern = f == SWEEP_STREAMED ? chain_stream_queue_kernel<T, T, true>
+                : f == SWEEP_STAGED ? chain_fwd_queue_kernel<T, true> : chain_fwd_queue_kernel<T, false>;
+    return queue_sweep<T>(kern, descs, items, nitems, head, smem, sms, s);
+}
+
 template <class T, class Tsep>
 cudaError_t queue_bwd(const SolveArgs<T> *descs, const WorkItem *items, int nitems, int *head, size_t smem, int sms,
-                      bool staged, cudaStream_t s)
+                      SweepForm f, cudaStream_t s)
 {
-    auto kern = staged ? chain_bwd_queue_kernel<T, Tsep, true> : chain_bwd_queue_kernel<T, Tsep, false>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    int per = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, SOLVE_THREADS, smem);
-    const int grid = std::max(1, std::min(nitems, sms * std::max(per, 1)));
-    e = cudaMemsetAsync(head, 0, sizeof(int), s);
-    if (e != cudaSuccess) return e;
-    kern<<<grid, SOLVE_THREADS, smem, s>>>(descs, items, nitems, head);
-    count_launch();
-    return cudaGetLastError();
+    auto kern = f == SWEEP_STREAMED ? chain_stream_queue_kernel<T, Tsep, false>
+                : f == SWEEP_STAGED ? chain_bwd_queue_kernel<T, Tsep, true> : chain_bwd_queue_kernel<T, Tsep, false>;
+    return queue_sweep<T>(kern, descs, items, nitems, head, smem, sms, s);
 }
 
 // ------------------------------------------------------------------ planning
@@ -266,10 +321,29 @@ void plan_factor_level(Builder &B, int level, bool coarsest)
         const size_t od = put_vec(B.blob, descs), oi = put_vec(B.blob, sorted), oh = B.blob.put(nullptr, 16);
         const int ni = (int)sorted.size();
         const int sms = b->sms;
+        size_t om = 0;
+        bool tma = true;
+        if constexpr (std::is_same<T, float>::value) {
+            if (nb == WIDE_CLASS + 1 && !coarsest) {
+                std::vector<CUtensorMap> maps(descs.size());
+                for (size_t q = 0; q < descs.size(); ++q)
+                    tma = (chain128_tmap_b<Tin>(descs[q], &maps[q]) || descs[q].n % 2 != 0) && tma;  // (odd n: plain loads)
+                om = put_vec(B.blob, maps);
+            }
+        }
         B.factor.push_back([=](char *base) {
             Step st;
             st.what = std::string("plan_factor_level") + " items=" + std::to_string(ni);
             st.run = [=](cudaStream_t s) {
+                if constexpr (std::is_same<T, float>::value) {
+                    if (nb == 64 && !coarsest)
+                        return queue_factor64_tc<Tin>((const ChainFactorArgs<Tin, T> *)(base + od),
+                                                      (const WorkItem *)(base + oi), ni, (int *)(base + oh), sms, s);
+                    if (nb == WIDE_CLASS + 1 && !coarsest)
+                        return queue_factor128_tc<Tin>((const ChainFactorArgs<Tin, T> *)(base + od),
+                                                       (const CUtensorMap *)(base + om), tma,
+                                                       (const WorkItem *)(base + oi), ni, (int *)(base + oh), sms, s);
+                }
                 return queue_factor<Tin, T>(nb, (const ChainFactorArgs<Tin, T> *)(base + od),
                                             (const WorkItem *)(base + oi), ni, (int *)(base + oh), sms, s);
             };
@@ -316,7 +390,7 @@ void plan_asm_schur(Builder &B, int level)
 
 // forward sweeps (and the coarsest level's full solve) of one level
 template <class T>
-void plan_fwd(Builder &B, int level, bool coarsest, bool staged, int nb, std::vector<std::function<Step(char *)>> &dst)
+void plan_fwd(Builder &B, int level, bool coarsest, SweepForm form, int nb, std::vector<std::function<Step(char *)>> &dst)
 {
     bss_batch *b = B.b;
     std::vector<SolveArgs<T>> descs;
@@ -330,10 +404,10 @@ void plan_fwd(Builder &B, int level, bool coarsest, bool staged, int nb, std::ve
         if (l >= L) continue;
         const Level &lv = h->levels[l];
         if (lv.seq != coarsest || (lv.t == F64) != std::is_same<T, double>::value) continue;
-        if (solve_staged<T>((int)h->n, (int)h->k) != staged || nb_class(h->n) != nb) continue;
+        if (sweep_form<T>(h, coarsest) != form || nb_class(h->n) != nb) continue;
         const int di = (int)descs.size();
         descs.push_back(make_solve_args<T>(h, l, 0, (int)h->k));
-        smem = std::max(smem, solve_smem_bytes<T>((int)h->n, (int)h->k, staged));
+        smem = std::max(smem, sweep_smem<T>(h, form));
         const long long q = lv.seq ? 1 : lv.Q;
         for (long long p = 0; p < q; ++p) {
             items.push_back(WorkItem{di, (int)p});
@@ -351,10 +425,10 @@ void plan_fwd(Builder &B, int level, bool coarsest, bool staged, int nb, std::ve
     const int sms = b->sms;
     dst.push_back([=](char *base) {
         Step st;
-        st.what = std::string("plan_fwd") + " items=" + std::to_string(ni) + " smem=" + std::to_string(smem) + (staged ? " staged" : " direct");
+        st.what = std::string("plan_fwd") + " items=" + std::to_string(ni) + " smem=" + std::to_string(smem) + sweep_name(form);
         st.run = [=](cudaStream_t s) {
             return queue_fwd<T>((const SolveArgs<T> *)(base + od), (const WorkItem *)(base + oi), ni,
-                                (int *)(base + oh), smem, sms, staged, s);
+                                (int *)(base + oh), smem, sms, form, s);
         };
         return st;
     });
@@ -396,7 +470,7 @@ void plan_asm_rhs(Builder &B, int level, std::vector<std::function<Step(char *)>
 }
 
 template <class T, class Tsep>
-void plan_bwd(Builder &B, int level, bool staged, int nb, std::vector<std::function<Step(char *)>> &dst)
+void plan_bwd(Builder &B, int level, SweepForm form, int nb, std::vector<std::function<Step(char *)>> &dst)
 {
     bss_batch *b = B.b;
     std::vector<SolveArgs<T>> descs;
@@ -409,10 +483,10 @@ void plan_bwd(Builder &B, int level, bool staged, int nb, std::vector<std::funct
         const Level &L = h->levels[level], &X = h->levels[level + 1];
         if ((L.t == F64) != std::is_same<T, double>::value || (X.t == F64) != std::is_same<Tsep, double>::value)
             continue;
-        if (solve_staged<T>((int)h->n, (int)h->k) != staged || nb_class(h->n) != nb) continue;
+        if (sweep_form<T>(h, false) != form || nb_class(h->n) != nb) continue;
         const int di = (int)descs.size();
         descs.push_back(make_solve_args<T>(h, level, 0, (int)h->k));
-        smem = std::max(smem, solve_smem_bytes<T>((int)h->n, (int)h->k, staged));
+        smem = std::max(smem, sweep_smem<T>(h, form));
         for (long long p = 0; p < L.Q; ++p) {
             items.push_back(WorkItem{di, (int)p});
             len.push_back((L.N - 1) / L.Q);
@@ -429,10 +503,10 @@ void plan_bwd(Builder &B, int level, bool staged, int nb, std::vector<std::funct
     const int sms = b->sms;
     dst.push_back([=](char *base) {
         Step st;
-        st.what = std::string("plan_bwd") + " items=" + std::to_string(ni) + " smem=" + std::to_string(smem) + (staged ? " staged" : " direct");
+        st.what = std::string("plan_bwd") + " items=" + std::to_string(ni) + " smem=" + std::to_string(smem) + sweep_name(form);
         st.run = [=](cudaStream_t s) {
             return queue_bwd<T, Tsep>((const SolveArgs<T> *)(base + od), (const WorkItem *)(base + oi), ni,
-                                      (int *)(base + oh), smem, sms, staged, s);
+                                      (int *)(base + oh), smem, sms, form, s);
         };
         return st;
     });
@@ -446,7 +520,7 @@ void plan_chain_solve(Builder &B, int maxpart, std::vector<std::function<Step(ch
     // would cap every CTA at the occupancy of the largest blocks
     static const int kClasses[] = {16, 32, 64, WIDE_CLASS};
     for (int l = 0; l < maxpart; ++l) {
-        for (bool st : {true, false})
+        for (SweepForm st : {SWEEP_STAGED, SWEEP_STREAMED, SWEEP_DIRECT})
             for (int nb : kClasses) {
                 plan_fwd<float>(B, l, false, st, nb, dst);
                 plan_fwd<double>(B, l, false, st, nb, dst);
@@ -455,13 +529,13 @@ void plan_chain_solve(Builder &B, int maxpart, std::vector<std::function<Step(ch
         plan_asm_rhs<float, double>(B, l, dst);
         plan_asm_rhs<double, double>(B, l, dst);
     }
-    for (bool st : {true, false})
+    for (SweepForm st : {SWEEP_STAGED, SWEEP_STREAMED, SWEEP_DIRECT})
         for (int nb : kClasses) {
             plan_fwd<float>(B, 0, true, st, nb, dst);
             plan_fwd<double>(B, 0, true, st, nb, dst);
         }
     for (int l = maxpart - 1; l >= 0; --l)
-        for (bool st : {true, false})
+        for (SweepForm st : {SWEEP_STAGED, SWEEP_STREAMED, SWEEP_DIRECT})
             for (int nb : kClasses) {
                 plan_bwd<float, float>(B, l, st, nb, dst);
                 plan_bwd<float, double>(B, l, st, nb, dst);

@@ -313,9 +313,16 @@ __device__ __forceinline__ bool c128_phase1(uint32_t tm, const float *rawW, cons
         });
 }
 
-template <class Tin>
+// QUEUE: the persistent form for many systems (see chain_factor_queue_kernel):
+// g and its tensor map come from descs and maps (with tma_b, all of them
+// valid), a CTA takes items until the queue is empty; otherwise the CTA walks
+// partitions blockIdx.x, + gridDim.x, ... of the argument (the grid is at
+// most one CTA per SM).
+template <class Tin, bool QUEUE>
 __global__ void __launch_bounds__(C128_THREADS, 1)
-    chain128_tc_kernel(ChainFactorArgs<Tin, float> g, const __grid_constant__ CUtensorMap tmB, int tma_b)
+    chain128_tc_kernel(ChainFactorArgs<Tin, float> g, const __grid_constant__ CUtensorMap tmB, int tma_b,
+                       const ChainFactorArgs<Tin, float> *__restrict__ descs, const CUtensorMap *__restrict__ maps,
+                       const WorkItem *__restrict__ items, int nitems, int *head)
 {
     constexpr int LD = C128_LD;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -335,13 +342,20 @@ __global__ void __launch_bounds__(C128_THREADS, 1)
     const int L = 32 * (w & 3) + lane;  // this thread's TMEM lane (accumulator row)
     const int cb = 64 * (w >> 2);       // its first accumulator column
     const uint32_t lane_base = (uint32_t)(32 * (w & 3)) << 16;
-    const int n = g.n;
-    const long long nn = (long long)n * n;
-    const bool aligned = ((uintptr_t)g.A_in % 16u) == 0 && ((uintptr_t)g.B_in % 16u) == 0;
+    int n = g.n;
+    long long nn = (long long)n * n;
     // bulk copies of column chunks (A) and the tensor copies of row chunks (B)
     // start on 16 bytes; the latter also need the 1024-byte-aligned buffers
-    const bool bulk = aligned && (sizeof(Tin) == 8 ? n % 2 == 0 : n % 4 == 0);
-    const bool tmab = sizeof(Tin) == 8 && bulk && tma_b != 0 && ((smem_u32(smem_raw) + C128_OFF_B) & 1023u) == 0;
+    bool bulk = false, tmab = false;
+    const CUtensorMap *map = &tmB;
+    auto set_system = [&]() {
+        n = g.n;
+        nn = (long long)n * n;
+        const bool aligned = ((uintptr_t)g.A_in % 16u) == 0 && ((uintptr_t)g.B_in % 16u) == 0;
+        bulk = aligned && (sizeof(Tin) == 8 ? n % 2 == 0 : n % 4 == 0);
+        tmab = sizeof(Tin) == 8 && bulk && tma_b != 0 && ((smem_u32(smem_raw) + C128_OFF_B) & 1023u) == 0;
+    };
+    if constexpr (!QUEUE) set_system();
 
     if (w == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
@@ -389,13 +403,29 @@ __global__ void __launch_bounds__(C128_THREADS, 1)
         if (tid == 64) {
             fence_async_smem();
             mbar_expect_tx(mb, (uint32_t)(16 * 128 * sizeof(Tin)));  // the whole box, zero-filled parts included
-            tma_load_2d(base_addr + (uint32_t)(C128_OFF_B + b * C128_BCH), &tmB, 16 * c, (int)(blk * n), mb);
+            tma_load_2d(base_addr + (uint32_t)(C128_OFF_B + b * C128_BCH), map, 16 * c, (int)(blk * n), mb);
         }
         if (tid == 0) b_pend |= 1u << b;
     };
 
-    // partitions p = blockIdx.x, + gridDim.x, ... (the grid is at most one CTA per SM)
-    for (long long p = blockIdx.x; p < g.Q && !*abort; p += gridDim.x) {
+    for (long long p = blockIdx.x; !*abort; p += gridDim.x) {
+    if constexpr (QUEUE) {
+        int *cur = reinterpret_cast<int *>(ctl + 1008);
+        if (tid == 0) *cur = atomicAdd(head, 1);
+        __syncthreads();
+        const int it = *cur;
+        __syncthreads();
+        if (it >= nitems) break;
+        const WorkItem item = items[it];
+        g = descs[item.desc];
+        p = item.p;
+        set_system();
+        map = maps + item.desc;
+        if (tid == 64 && tmab)  // the map was written outside this kernel's tensor-map proxy
+            asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(map) : "memory");
+    } else {
+        if (p >= g.Q) break;
+    }
     const long long sL = (p * (g.N - 1)) / g.Q;
     const long long sR = ((p + 1) * (g.N - 1)) / g.Q;
     const long long first = sL + 1, last = sR - 1;

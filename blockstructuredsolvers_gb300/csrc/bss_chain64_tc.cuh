@@ -171,8 +171,13 @@ __device__ __forceinline__ void c64_workers_sync() { asm volatile("bar.sync 2, 2
 constexpr int C64_AREG = (64 * 64 + 223) / 224;  // A_i elements per converter thread: 19
 constexpr int C64_BREG = (16 * 64 + 223) / 224;  // B_i 4-element groups per converter thread: 5
 
-template <class Tin>
-__global__ void __launch_bounds__(C64_THREADS, 2) chain64_tc_kernel(ChainFactorArgs<Tin, float> g)
+// QUEUE: the persistent form for many systems (see chain_factor_queue_kernel):
+// g comes from descs, a CTA takes items until the queue is empty; otherwise g
+// is the argument and a CTA's partition its index.
+template <class Tin, bool QUEUE>
+__global__ void __launch_bounds__(C64_THREADS, 2)
+    chain64_tc_kernel(ChainFactorArgs<Tin, float> g, const ChainFactorArgs<Tin, float> *__restrict__ descs,
+                      const WorkItem *__restrict__ items, int nitems, int *head)
 {
     constexpr int LD = Geo<float, 64>::LD;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -194,14 +199,6 @@ __global__ void __launch_bounds__(C64_THREADS, 2) chain64_tc_kernel(ChainFactorA
     const int L = 32 * (w & 3) + lane;  // this thread's TMEM lane (accumulator row)
     const int c0 = 32 * (w >> 2);       // its first accumulator column
     const uint32_t lane_base = (uint32_t)(32 * (w & 3)) << 16;
-    const int n = g.n;
-    const long long nn = (long long)n * n;
-    const long long p = blockIdx.x;
-    const long long sL = (p * (g.N - 1)) / g.Q;
-    const long long sR = ((p + 1) * (g.N - 1)) / g.Q;
-    const long long first = sL + 1, last = sR - 1;
-    const uint32_t blk_bytes = (uint32_t)(nn * (long long)sizeof(Tin));
-    const bool bulk = (blk_bytes % 16u) == 0 && ((uintptr_t)g.A_in % 16u) == 0 && ((uintptr_t)g.B_in % 16u) == 0;
 
     if (w == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
@@ -223,7 +220,29 @@ __global__ void __launch_bounds__(C64_THREADS, 2) chain64_tc_kernel(ChainFactorA
     const uint32_t sRa = smem_u32(R), sVa = smem_u32(VR);
     C64Bar bM{smem_u32(&mbars[0]), 0u, false}, bA{smem_u32(&mbars[1]), 0u, false}, bB{smem_u32(&mbars[2]), 0u, false};
 
+    for (;;) {  // items
+    long long p = blockIdx.x;
+    if constexpr (QUEUE) {
+        int *cur = reinterpret_cast<int *>(tail + 12);
+        if (tid == 0) *cur = atomicAdd(head, 1);
+        __syncthreads();
+        const int it = *cur;
+        __syncthreads();
+        if (it >= nitems) break;
+        const WorkItem item = items[it];
+        g = descs[item.desc];
+        p = item.p;
+    }
+    const int n = g.n;
+    const long long nn = (long long)n * n;
+    const long long sL = (p * (g.N - 1)) / g.Q;
+    const long long sR = ((p + 1) * (g.N - 1)) / g.Q;
+    const long long first = sL + 1, last = sR - 1;
+    const uint32_t blk_bytes = (uint32_t)(nn * (long long)sizeof(Tin));
+    const bool bulk = (blk_bytes % 16u) == 0 && ((uintptr_t)g.A_in % 16u) == 0 && ((uintptr_t)g.B_in % 16u) == 0;
+
     if (first <= last && bulk && tid == 32) {
+        fence_async_smem();  // (an earlier item's generic accesses of the copy's target)
         mbar_expect_tx(bA.addr, blk_bytes);
         bulk_g2s(sVa, g.A_in + first * nn, blk_bytes, bA.addr);
         bA.pending = true;
@@ -483,7 +502,10 @@ __global__ void __launch_bounds__(C64_THREADS, 2) chain64_tc_kernel(ChainFactorA
                 if (c0 + q < n) Cp[r + (long long)(c0 + q) * n] = dv[q];
         }
     }
+    tc_fence_before();
     __syncthreads();
+    if (!QUEUE || *abort) break;
+    }  // items
     if (*abort) {
         // a wait gave up: wait (bounded) for this CTA's MMAs (thread 0) and
         // copies (thread 32) still in flight before its shared memory and

@@ -51,10 +51,11 @@ namespace bss {
 // ---------------------------------------------------------------------------
 struct DevStatus {
     unsigned long long bad_key;  // min over ((level << 40) | block) of failed pivots
+    unsigned long long anorm;    // FP64 bits of ||T||_inf
+    // rnorm .. iters are cleared together when a solve begins
     unsigned long long rnorm;    // FP64 bits of max |r| (non-negative doubles order as ints)
     unsigned long long xnorm;    // FP64 bits of max |x|
     unsigned long long dnorm;    // FP64 bits of max |d|
-    unsigned long long anorm;    // FP64 bits of ||T||_inf
     double relres;
     int done;
     int iters;        // refinement corrections applied by the last solve
@@ -2414,6 +2415,29 @@ __global__ void absmax_kernel(const T *__restrict__ v, long long count, unsigned
     if ((threadIdx.x & 31) == 0) atomic_max_nonneg(dst, best);
 }
 
+// the start of a mixed solve: c = d rounded to the factors' type, *dst = max |d|
+// (as bits, which order like the numbers: an FP64 maximum is an FP64-pipe
+// instruction); NaN is ignored, as fmax ignores it
+template <class Tc>
+__global__ void rhs_begin_kernel(Tc *__restrict__ c, const double *__restrict__ d, long long count,
+                                 unsigned long long *dst)
+{
+    constexpr unsigned long long INF = 0x7FF0000000000000ull;
+    unsigned long long best = 0;
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < count;
+         e += (long long)gridDim.x * blockDim.x) {
+        const double v = d[e];
+        c[e] = (Tc)v;
+        const unsigned long long m = (unsigned long long)__double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFull;
+        if (m <= INF && m > best) best = m;
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long x = __shfl_xor_sync(0xffffffffu, best, o);
+        best = x > best ? x : best;
+    }
+    if ((threadIdx.x & 31) == 0) atomicMax(dst, best);
+}
+
 // r = d - T x in FP64 over the block-tridiagonal operator.  The FP64 FMA
 // pipe (~2 per clock per SM on GB300) bounds this kernel, not HBM, so it is
 // shaped to keep that pipe fed: several small CTAs per SM, each owning a
@@ -3078,6 +3102,8 @@ static __global__ void relres_control_kernel(DevStatus *st, double tol, int max_
         st->relres = rel;
         st->done = done;
         st->need_anorm = 0;
+        st->rnorm = 0ULL;  // for the next residual
+        st->xnorm = 0ULL;
         if (cont) {
             st->iters += 1;
             st->iters_total += 1;
@@ -3098,6 +3124,21 @@ static __global__ void relres_kernel(DevStatus *st, double tol)
         const double rel = den > 0.0 ? rn / den : 0.0;
         st->relres = rel;
         st->done = (rel <= tol) ? 1 : 0;
+        st->need_anorm = 0;
+        st->rnorm = 0ULL;  // for the next residual
+        st->xnorm = 0ULL;
+    }
+}
+
+// status words at the start of a factorization: no failed pivot, no expired
+// wait; mixed precision: ||T||_inf to be formed by the first residual
+static __global__ void factor_status_kernel(DevStatus *st, int mixed)
+{
+    st->bad_key = ~0ULL;
+    st->tc_timeout = 0;
+    if (mixed) {
+        st->anorm = 0ULL;
+        st->need_anorm = 1;
     }
 }
 
@@ -3256,14 +3297,6 @@ __global__ void update_kernel(double *__restrict__ x, const Tc *__restrict__ c, 
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < count;
          e += (long long)gridDim.x * blockDim.x)
         x[e] = assign ? (double)c[e] : x[e] + (double)c[e];
-}
-
-template <class Ts, class Td>
-__global__ void convert_kernel(Td *__restrict__ dst, const Ts *__restrict__ src, long long count)
-{
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < count;
-         e += (long long)gridDim.x * blockDim.x)
-        dst[e] = (Td)src[e];
 }
 
 template <class T>

@@ -22,6 +22,10 @@ template <class Tin, class T>
 cudaError_t launch_chain_factor(const ChainFactorArgs<Tin, T> &a, cudaStream_t s);
 template <class Tin, class T>
 int chain_factor_ctas_per_sm(int n, int variant);
+// the tensor map of a level's B blocks that chain128_tc_kernel reads them
+// with; false when they do not qualify
+template <class Tin>
+bool chain128_tmap_b(const ChainFactorArgs<Tin, float> &a, CUtensorMap *map);
 
 // FACTOR_* variant bits that handles take when the autotuner has no entry
 // for their (n, dtype, precision); process-wide
@@ -56,13 +60,15 @@ cudaError_t launch_residual(const T *A, const T *B, const T *x, const T *d, Tr *
 template <class Tr>
 cudaError_t launch_residual_df(const double *A, const double *B, const double *x, const double *d, Tr *r,
                                long long N, int n, int k, int with_norm, DevStatus *st, cudaStream_t s);
+// start of a factorization / of a mixed solve (c0 = d, max |d|, norms cleared)
+cudaError_t launch_factor_status(DevStatus *st, int mixed, cudaStream_t s);
+template <class Tc>
+cudaError_t launch_rhs_begin(Tc *c, const double *d, long long count, DevStatus *st, cudaStream_t s);
 cudaError_t launch_relres(DevStatus *st, double tol, cudaStream_t s);
 cudaError_t launch_relres_control(DevStatus *st, double tol, int max_refine, cudaGraphConditionalHandle hloop,
                                   cudaGraphConditionalHandle hcorr, cudaStream_t s);
 template <class Tc>
 cudaError_t launch_update(double *x, const Tc *c, long long count, int assign, cudaStream_t s);
-template <class Ts, class Td>
-cudaError_t launch_convert(Td *dst, const Ts *src, long long count, cudaStream_t s);
 template <class T>
 cudaError_t launch_init_identity(T *A, long long first_blk, long long last_blk, int n, cudaStream_t s);
 

@@ -1,6 +1,7 @@
 // Launcher definitions, included by the per-dtype kernel translation units.
 #pragma once
 
+#include <cstddef>
 #include <cstring>
 
 #include "bss_launch.h"
@@ -21,11 +22,11 @@ template <class Tin>
 static cudaError_t chain64_tc(const ChainFactorArgs<Tin, float> &a, cudaStream_t s)
 {
     const size_t smem = chain64_tc_smem();
-    auto kern = chain64_tc_kernel<Tin>;
+    auto kern = chain64_tc_kernel<Tin, false>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    kern<<<(unsigned)a.Q, C64_THREADS, smem, s>>>(a);
+    kern<<<(unsigned)a.Q, C64_THREADS, smem, s>>>(a, nullptr, nullptr, 0, nullptr);
     count_launch();
     return cudaGetLastError();
 }
@@ -138,7 +139,7 @@ static cudaError_t chain128_tc(const ChainFactorArgs<Tin, float> &a, cudaStream_
     const size_t smem = chain128_tc_smem();
     CUtensorMap tmB;
     const int tma_b = chain128_tmap_b<Tin>(a, &tmB) ? 1 : 0;
-    auto kern = chain128_tc_kernel<Tin>;
+    auto kern = chain128_tc_kernel<Tin, false>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
@@ -146,7 +147,7 @@ static cudaError_t chain128_tc(const ChainFactorArgs<Tin, float> &a, cudaStream_
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const unsigned grid = (unsigned)(a.Q < sms ? a.Q : sms);  // one CTA per SM walks several partitions
-    kern<<<grid, C128_THREADS, smem, s>>>(a, tmB, tma_b);
+    kern<<<grid, C128_THREADS, smem, s>>>(a, tmB, tma_b, nullptr, nullptr, nullptr, 0, nullptr);
     count_launch();
     return cudaGetLastError();
 }
@@ -196,7 +197,7 @@ static int ctas_nb(int variant)
     if constexpr (std::is_same<T, float>::value && NB == 64) {
         if (!(variant & FACTOR_FMA_CHAIN)) {
             const size_t smem = chain64_tc_smem();
-            auto kern = chain64_tc_kernel<Tin>;
+            auto kern = chain64_tc_kernel<Tin, false>;
             if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
                 return 1;
             cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
@@ -458,10 +459,12 @@ cudaError_t launch_update(double *x, const Tc *c, long long count, int assign, c
     return cudaGetLastError();
 }
 
-template <class Ts, class Td>
-cudaError_t launch_convert(Td *dst, const Ts *src, long long count, cudaStream_t s)
+template <class Tc>
+cudaError_t launch_rhs_begin(Tc *c, const double *d, long long count, DevStatus *st, cudaStream_t s)
 {
-    convert_kernel<Ts, Td><<<grid_for(count, 256), 256, 0, s>>>(dst, src, count);
+    cudaError_t e = cudaMemsetAsync(&st->rnorm, 0, offsetof(DevStatus, need_anorm) - offsetof(DevStatus, rnorm), s);
+    if (e != cudaSuccess) return e;
+    rhs_begin_kernel<Tc><<<grid_for(count, 256), 256, 0, s>>>(c, d, count, &st->dnorm);
     count_launch();
     return cudaGetLastError();
 }

@@ -42,48 +42,52 @@ struct KfScratch {
     }
 };
 
-// one CTA: the per-model blocks (O(n^3) once per model)
-__global__ void kf_prepare_kernel(int n, int m, const double *F, const double *H, const double *Qinv,
+// The per-model blocks (O(n^3) once per model) in two grids, one element a
+// thread: QF, RH and P0^{-1} x0, then the blocks of the normal equations from
+// them.  On GB300's FP64 pipe one CTA took 180 us for n = 64; spread over the
+// SMs a grid is a column of FMAs long (@@).
+__global__ void kf_factors_kernel(int n, int m, const double *F, const double *H, const double *Qinv,
                                   const double *Rinv, const double *P0inv, const double *x0, KfScratch w)
 {
-    const int nn = n * n;
-    for (int e = threadIdx.x; e < nn; e += blockDim.x) {  // QF = Q^{-1} F
+    const int e = blockIdx.x * blockDim.x + threadIdx.x, nn = n * n;
+    if (e < nn) {  // QF = Q^{-1} F
         const int r = e % n, c = e / n;
         double s = 0.0;
+#pragma unroll 8
         for (int j = 0; j < n; ++j) s = fma(Qinv[r + j * n], F[j + c * n], s);
         w.QF[e] = s;
-    }
-    for (int e = threadIdx.x; e < m * n; e += blockDim.x) {  // RH = R^{-1} H
-        const int r = e % m, c = e / m;
+    } else if (e < nn + m * n) {  // RH = R^{-1} H
+        const int q = e - nn, r = q % m, c = q / m;
         double s = 0.0;
+#pragma unroll 8
         for (int j = 0; j < m; ++j) s = fma(Rinv[r + j * m], H[j + c * m], s);
-        w.RH[e] = s;
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < nn; e += blockDim.x) {  // F^T Q^{-1} F and H^T R^{-1} H
-        const int r = e % n, c = e / n;
-        double s = 0.0, t = 0.0;
-        for (int j = 0; j < n; ++j) s = fma(F[j + r * n], w.QF[j + c * n], s);
-        for (int j = 0; j < m; ++j) t = fma(H[j + r * m], w.RH[j + c * m], t);
-        w.FQF[e] = s;
-        w.HRH[e] = t;
-    }
-    for (int e = threadIdx.x; e < n; e += blockDim.x) {
+        w.RH[q] = s;
+    } else if (e < nn + m * n + n) {
+        const int r = e - nn - m * n;
         double s = 0.0;
         if (P0inv && x0)
-            for (int j = 0; j < n; ++j) s = fma(P0inv[e + j * n], x0[j], s);
-        w.p0x[e] = s;
+            for (int j = 0; j < n; ++j) s = fma(P0inv[r + j * n], x0[j], s);
+        w.p0x[r] = s;
     }
-    __syncthreads();
-    for (int e = threadIdx.x; e < nn; e += blockDim.x) {
-        const int r = e % n, c = e / n;
-        const int u = r <= c ? e : c + r * n;  // upper-triangle source (Symmetric(Akk))
-        const double hrh = w.HRH[u], fqf = w.FQF[u], qi = Qinv[u];
-        w.Aint[e] = hrh + qi + fqf;
-        w.Afirst[e] = P0inv ? hrh + P0inv[u] + fqf : hrh + qi + fqf;
-        w.Alast[e] = P0inv ? hrh + qi : hrh + qi + fqf;
-        w.Bup[e] = -w.QF[c + r * n];  // -(Q^{-1} F)^T
-    }
+}
+
+__global__ void kf_blocks_kernel(int n, int m, const double *F, const double *H, const double *Qinv,
+                                 const double *P0inv, KfScratch w)
+{
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= n * n) return;
+    const int r0 = e % n, c0 = e / n;
+    const int r = min(r0, c0), c = max(r0, c0), u = r + c * n;  // upper-triangle source (Symmetric(Akk))
+    double fqf = 0.0, hrh = 0.0;                               // F^T Q^{-1} F, H^T R^{-1} H
+#pragma unroll 8
+    for (int j = 0; j < n; ++j) fqf = fma(F[j + r * n], w.QF[j + c * n], fqf);
+#pragma unroll 8
+    for (int j = 0; j < m; ++j) hrh = fma(H[j + r * m], w.RH[j + c * m], hrh);
+    const double qi = Qinv[u];
+    w.Aint[e] = hrh + qi + fqf;
+    w.Afirst[e] = P0inv ? hrh + P0inv[u] + fqf : hrh + qi + fqf;
+    w.Alast[e] = P0inv ? hrh + qi : hrh + qi + fqf;
+    w.Bup[e] = -w.QF[c0 + r0 * n];  // -(Q^{-1} F)^T
 }
 
 __global__ void kf_fill_ab_kernel(long long N, int n, KfScratch w, double *A, double *B)
@@ -122,7 +126,9 @@ cudaError_t kf_launch_prepare(long long n, long long m, const double *F, const d
                               const double *Rinv, const double *P0inv, const double *x0, const KfScratch &w,
                               cudaStream_t s)
 {
-    kf_prepare_kernel<<<1, 256, 0, s>>>((int)n, (int)m, F, H, Qinv, Rinv, P0inv, x0, w);
+    kf_factors_kernel<<<(unsigned)((n * n + m * n + n + 63) / 64), 64, 0, s>>>((int)n, (int)m, F, H, Qinv, Rinv, P0inv, x0, w);
+    count_launch();
+    kf_blocks_kernel<<<(unsigned)((n * n + 63) / 64), 64, 0, s>>>((int)n, (int)m, F, H, Qinv, P0inv, w);
     count_launch();
     return cudaGetLastError();
 }

@@ -87,38 +87,69 @@ __device__ __forceinline__ bool ring_wait(StreamRing &rg, int q)
 // quarter-warp share column c, lane `part` takes the vector chunks part,
 // part + 8, ... of the column (so a quarter-warp reads 128 contiguous bytes
 // of M and of v per step: no bank conflicts), multiplies each with all four
-// v columns, and a 3-level shuffle sums the 8 parts. qc is a multiple of 4,
-// so whole warps leave together.
-template <class T>
-__device__ __forceinline__ void slot_tmul8(const T *sM, int qc, const T *v, T *out, int c0, int n, int kc, T sign,
-                                           bool accumulate)
+// v columns, and shuffles sum the 8 parts. qc is a multiple of 4, so whole
+// warps leave together.  Rows from `rows` on are zero (V: below the slot's
+// last column).
+template <class T, int JT>
+__device__ __forceinline__ void slot_tmul8_j(const T *sM, int qc, const T *v, T *out, int c0, int n, int kc, T sign,
+                                             bool accumulate, int rows)
 {
     using VT = typename Vec<T>::type;
     constexpr int W = Vec<T>::W;
     const int part = threadIdx.x & 7, c = threadIdx.x >> 3;
     if (c >= qc) return;
     const T *mc = sM + (size_t)c * n;
-    for (int j0 = 0; j0 < kc; j0 += 4) {
-        T acc[4] = {T(0), T(0), T(0), T(0)};
-        for (int r = part * W; r < n; r += 8 * W) {
+    for (int j0 = 0; j0 < kc; j0 += JT) {
+        T acc[JT];
+#pragma unroll
+        for (int q = 0; q < JT; ++q) acc[q] = T(0);
+#pragma unroll 4
+        for (int r = part * W; r < rows; r += 8 * W) {
             const VT m = *reinterpret_cast<const VT *>(mc + r);
 #pragma unroll
-            for (int q = 0; q < 4; ++q)
-                if (j0 + q < kc) fma_vec(acc[q], m, *reinterpret_cast<const VT *>(v + r + (size_t)(j0 + q) * n));
+            for (int q = 0; q < JT; ++q) {
+                // columns beyond the last: repeated in FP32 (no branch between the
+                // reads), skipped in FP64 (whose FMAs are the bound)
+                if (sizeof(T) == 4 || j0 + q < kc)
+                    fma_vec(acc[q], m, *reinterpret_cast<const VT *>(v + r + (size_t)min(j0 + q, kc - 1) * n));
+            }
         }
+        // the 8 shares' sums, each lane keeping half of the columns while there are two or more
+        int j = 0;
+        if constexpr (JT == 4) {
+            const bool up = (part & 4) != 0;
 #pragma unroll
-        for (int o = 4; o > 0; o >>= 1)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
-        if (part == 0) {
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-                if (j0 + q < kc) {
-                    const int oo = c0 + c + (j0 + q) * n;
-                    out[oo] = accumulate ? out[oo] + sign * acc[q] : sign * acc[q];
-                }
+            for (int q = 0; q < 2; ++q) {
+                const T send = up ? acc[q] : acc[q + 2], keep = up ? acc[q + 2] : acc[q];
+                acc[q] = keep + __shfl_xor_sync(0xffffffffu, send, 4);
+            }
+            j = up ? 2 : 0;
+        } else if constexpr (JT == 1) {
+            acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 4);
+        }
+        if constexpr (JT >= 2) {
+            constexpr int B = JT == 4 ? 2 : 4;
+            const bool up = (part & B) != 0;
+            const T send = up ? acc[0] : acc[1], keep = up ? acc[1] : acc[0];
+            acc[0] = keep + __shfl_xor_sync(0xffffffffu, send, B);
+            j += up ? 1 : 0;
+        }
+        if constexpr (JT <= 2) acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 2);
+        acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 1);
+        constexpr int IDLE = JT == 4 ? 1 : JT == 2 ? 3 : 7;
+        if ((part & IDLE) == 0 && j0 + j < kc) {
+            const int oo = c0 + c + (j0 + j) * n;
+            out[oo] = accumulate ? out[oo] + sign * acc[0] : sign * acc[0];
         }
     }
+}
+template <class T>
+__device__ __forceinline__ void slot_tmul8(const T *sM, int qc, const T *v, T *out, int c0, int n, int kc, T sign,
+                                           bool accumulate, int rows)
+{
+    if (kc == 1) slot_tmul8_j<T, 1>(sM, qc, v, out, c0, n, kc, sign, accumulate, rows);
+    else if (kc == 2) slot_tmul8_j<T, 2>(sM, qc, v, out, c0, n, kc, sign, accumulate, rows);
+    else slot_tmul8_j<T, 4>(sM, qc, v, out, c0, n, kc, sign, accumulate, rows);
 }
 
 // Backward product mapping: thread (rg, jg, part) owns rows 4 rg .. 4 rg + 3
@@ -234,12 +265,17 @@ __device__ __forceinline__ bool ring_pass(StreamRing &rg, T *ring, int qelems, c
     return true;
 }
 
-template <class T>
-__device__ __forceinline__ void ring_setup(StreamRing &rg, T *ring, uint64_t *bars, int *abort, int n)
+// shared memory: 4 mbarriers and the abort flag (64 bytes), then the ring
+constexpr int STREAM_HEAD = 64;
+
+__device__ __forceinline__ void ring_setup(StreamRing &rg)
 {
-    rg.base = smem_u32(ring);
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem_raw);
+    int *abort = reinterpret_cast<int *>(bars + 4);
+    rg.base = smem_u32(smem_raw + STREAM_HEAD);
     rg.bars = smem_u32(bars);
-    rg.qbytes = (uint32_t)((size_t)n * n / 4 * sizeof(T));
+    rg.qbytes = 0u;
     rg.phase = 0u;
     rg.pending = 0u;
     if (threadIdx.x == 0) {
@@ -263,25 +299,25 @@ __device__ __forceinline__ void ring_abort(StreamRing &rg, DevStatus *st)
 // forward sweep of partition p: y_i = V_i^T (d_i - W_{i-1}^T y_{i-1}),
 // bL = sum Y_i^T y_i, bR = W_last^T y_last (as chain_fwd_body)
 template <class T>
-__device__ __forceinline__ void chain_fwd_stream_body(const SolveArgs<T> &g, const long long p)
+__device__ __forceinline__ void chain_fwd_stream_body(const SolveArgs<T> &g, const long long p, StreamRing &rg)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int n = g.n, kc = g.kc;
     const int nn = n * n, nkc = n * kc, qelems = nn / 4, qc = n / 4;
-    T *ring = reinterpret_cast<T *>(smem_raw);
+    T *ring = reinterpret_cast<T *>(smem_raw + STREAM_HEAD);
     T *sr = ring + nn;
     T *sy = sr + nkc;
     T *sbL = sy + nkc;
     T *sbR = sbL + nkc;
-    uint64_t *bars = reinterpret_cast<uint64_t *>(sbR + nkc + 2 * nkc);
-    int *abort = reinterpret_cast<int *>(bars + 4);
+    int *abort = reinterpret_cast<int *>(smem_raw + 32);
     const long long sL = (p * (g.N - 1)) / g.Q;
     const long long sR = ((p + 1) * (g.N - 1)) / g.Q;
     const long long first = sL + 1, last = sR - 1;
-    StreamRing rg;
-    ring_setup<T>(rg, ring, bars, abort, n);
-    if (threadIdx.x == 0)
+    rg.qbytes = (uint32_t)(qelems * (int)sizeof(T));
+    if (threadIdx.x == 0) {
+        fence_async_smem();
         for (int q = 0; q < 4; ++q) ring_issue<T>(rg, g.Af + first * (long long)nn, q, qelems);
+    }
     for (int e = threadIdx.x; e < nkc; e += blockDim.x) sbL[e] = T(0);
     for (long long i = first; i <= last; ++i) {
         if (threadIdx.x == 64 && i < last)
@@ -291,24 +327,24 @@ __device__ __forceinline__ void chain_fwd_stream_body(const SolveArgs<T> &g, con
             __syncthreads();
             // sr -= W_{i-1}^T y_{i-1}; the ring holds W_{i-1}, then V_i
             if (!ring_pass<T>(rg, ring, qelems, g.Af + i * (long long)nn, g.Y + i * (long long)nn, abort,
-                              [&](int q, const T *slot) { slot_tmul8<T>(slot, qc, sy, sr, q * qc, n, kc, T(-1), true); }))
+                              [&](int q, const T *slot) { slot_tmul8<T>(slot, qc, sy, sr, q * qc, n, kc, T(-1), true, n); }))
                 return ring_abort(rg, g.st);
         }
         __syncthreads();
         // y_i = V_i^T sr; then Y_i
         if (!ring_pass<T>(rg, ring, qelems, g.Y + i * (long long)nn, g.Bf + i * (long long)nn, abort,
-                          [&](int q, const T *slot) { slot_tmul8<T>(slot, qc, sr, sy, q * qc, n, kc, T(1), false); }))
+                          [&](int q, const T *slot) { slot_tmul8<T>(slot, qc, sr, sy, q * qc, n, kc, T(1), false, (q + 1) * qc); }))
             return ring_abort(rg, g.st);
         // bL += Y_i^T y_i; then W_i (the next step's W_{i-1}, or W_last)
         const T *after = i < last ? g.Af + (i + 1) * (long long)nn : (const T *)nullptr;
         if (!ring_pass<T>(rg, ring, qelems, g.Bf + i * (long long)nn, after, abort,
-                          [&](int q, const T *slot) { slot_tmul8<T>(slot, qc, sy, sbL, q * qc, n, kc, T(1), true); }))
+                          [&](int q, const T *slot) { slot_tmul8<T>(slot, qc, sy, sbL, q * qc, n, kc, T(1), true, n); }))
             return ring_abort(rg, g.st);
         store_rhs(g.d, sy, i, n, g.k, g.j0, kc);
     }
     // bR = W_last^T y_last
     if (!ring_pass<T>(rg, ring, qelems, (const T *)nullptr, (const T *)nullptr, abort,
-                      [&](int q, const T *slot) { slot_tmul8<T>(slot, qc, sy, sbR, q * qc, n, kc, T(1), false); }))
+                      [&](int q, const T *slot) { slot_tmul8<T>(slot, qc, sy, sbR, q * qc, n, kc, T(1), false, n); }))
         return ring_abort(rg, g.st);
     T *bp = g.bvec + p * 2 * (long long)nkc;
     for (int e = threadIdx.x; e < nkc; e += blockDim.x) {
@@ -320,27 +356,27 @@ __device__ __forceinline__ void chain_fwd_stream_body(const SolveArgs<T> &g, con
 // backward sweep of partition p: x_i = V_i (y_i - Y_i x_L - W_i x_{i+1})
 // with x_{last+1} = x_R (as chain_bwd_body); separators copied from xsep
 template <class T, class Tsep>
-__device__ __forceinline__ void chain_bwd_stream_body(const SolveArgs<T> &g, const long long p)
+__device__ __forceinline__ void chain_bwd_stream_body(const SolveArgs<T> &g, const long long p, StreamRing &rg)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int n = g.n, kc = g.kc;
     const int nn = n * n, nkc = n * kc, qelems = nn / 4, qc = n / 4;
-    T *ring = reinterpret_cast<T *>(smem_raw);
+    T *ring = reinterpret_cast<T *>(smem_raw + STREAM_HEAD);
     T *sz = ring + nn;
     T *sxL = sz + nkc;
     T *sxn = sxL + nkc;
     T *sxt = sxn + nkc;
     T *red = sxt + 3 * nkc;  // STREAM_PARTIAL elements
-    uint64_t *bars = reinterpret_cast<uint64_t *>(red + STREAM_PARTIAL);
-    int *abort = reinterpret_cast<int *>(bars + 4);
+    int *abort = reinterpret_cast<int *>(smem_raw + 32);
     const long long sL = (p * (g.N - 1)) / g.Q;
     const long long sR = ((p + 1) * (g.N - 1)) / g.Q;
     const long long first = sL + 1, last = sR - 1;
     const Tsep *xs = reinterpret_cast<const Tsep *>(g.xsep);
-    StreamRing rg;
-    ring_setup<T>(rg, ring, bars, abort, n);
-    if (threadIdx.x == 0)
+    rg.qbytes = (uint32_t)(qelems * (int)sizeof(T));
+    if (threadIdx.x == 0) {
+        fence_async_smem();
         for (int q = 0; q < 4; ++q) ring_issue<T>(rg, g.Y + last * (long long)nn, q, qelems);
+    }
     load_rhs(sxL, xs, p, n, g.k, g.j0, kc);
     load_rhs(sxn, xs, p + 1, n, g.k, g.j0, kc);
     __syncthreads();
@@ -381,13 +417,45 @@ __device__ __forceinline__ void chain_bwd_stream_body(const SolveArgs<T> &g, con
 template <class T>
 __global__ void __launch_bounds__(SOLVE_THREADS) chain_fwd_stream_kernel(SolveArgs<T> g)
 {
-    chain_fwd_stream_body<T>(g, blockIdx.x);
+    StreamRing rg;
+    ring_setup(rg);
+    chain_fwd_stream_body<T>(g, blockIdx.x, rg);
 }
 
 template <class T, class Tsep>
 __global__ void __launch_bounds__(SOLVE_THREADS) chain_bwd_stream_kernel(SolveArgs<T> g)
 {
-    chain_bwd_stream_body<T, Tsep>(g, blockIdx.x);
+    StreamRing rg;
+    ring_setup(rg);
+    chain_bwd_stream_body<T, Tsep>(g, blockIdx.x, rg);
+}
+
+// the persistent forms for many systems (see chain_factor_queue_kernel);
+// Tsep unused by the forward sweep
+template <class T, class Tsep, bool FWD>
+__global__ void __launch_bounds__(SOLVE_THREADS)
+    chain_stream_queue_kernel(const SolveArgs<T> *__restrict__ descs, const WorkItem *__restrict__ items, int nitems,
+                              int *head)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ int cur;
+    StreamRing rg;
+    ring_setup(rg);
+    for (;;) {
+        if (threadIdx.x == 0) cur = atomicAdd(head, 1);
+        __syncthreads();
+        const int it = cur;
+        __syncthreads();
+        if (it >= nitems) break;
+        const WorkItem w = items[it];
+        const SolveArgs<T> g = descs[w.desc];
+        if constexpr (FWD)
+            chain_fwd_stream_body<T>(g, w.p, rg);
+        else
+            chain_bwd_stream_body<T, Tsep>(g, w.p, rg);
+        __syncthreads();
+        if (*reinterpret_cast<int *>(smem_raw + 32)) break;
+    }
 }
 
 }  // namespace bss

@@ -5,6 +5,7 @@
 namespace bss {
 template cudaError_t launch_chain_factor<float, float>(const ChainFactorArgs<float, float> &, cudaStream_t);
 template int chain_factor_ctas_per_sm<float, float>(int, int);
+template bool chain128_tmap_b<float>(const ChainFactorArgs<float, float> &, CUtensorMap *);
 template cudaError_t launch_assemble_schur<float, float, float>(const float *, const float *, float *, float *,
                                                                 long long, long long, int, cudaStream_t);
 template cudaError_t launch_assemble_schur<float, float, double>(const float *, const float *, double *, double *,
@@ -22,6 +23,5 @@ template cudaError_t launch_absmax<float>(const float *, long long, unsigned lon
 template cudaError_t launch_residual<float, float>(const float *, const float *, const float *, const float *,
                                                    float *, long long, int, int, int, DevStatus *, cudaStream_t);
 template cudaError_t launch_update<float>(double *, const float *, long long, int, cudaStream_t);
-template cudaError_t launch_convert<float, double>(double *, const float *, long long, cudaStream_t);
 template cudaError_t launch_init_identity<float>(float *, long long, long long, int, cudaStream_t);
 }  // namespace bss

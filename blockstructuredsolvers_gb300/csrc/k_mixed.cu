@@ -7,6 +7,7 @@
 namespace bss {
 template cudaError_t launch_chain_factor<double, float>(const ChainFactorArgs<double, float> &, cudaStream_t);
 template int chain_factor_ctas_per_sm<double, float>(int, int);
+template bool chain128_tmap_b<double>(const ChainFactorArgs<double, float> &, CUtensorMap *);
 template cudaError_t launch_assemble_schur<double, float, float>(const double *, const float *, float *, float *,
                                                                  long long, long long, int, cudaStream_t);
 template cudaError_t launch_assemble_schur<double, float, double>(const double *, const float *, double *,
@@ -19,14 +20,21 @@ template cudaError_t launch_residual_df<float>(const double *, const double *, c
                                                float *, long long, int, int, int, DevStatus *, cudaStream_t);
 template cudaError_t launch_residual_df<double>(const double *, const double *, const double *, const double *,
                                                 double *, long long, int, int, int, DevStatus *, cudaStream_t);
-template cudaError_t launch_convert<double, float>(float *, const double *, long long, cudaStream_t);
-template cudaError_t launch_convert<double, double>(double *, const double *, long long, cudaStream_t);
-template cudaError_t launch_convert<float, float>(float *, const float *, long long, cudaStream_t);
 
 static std::atomic<long long> g_launches{0};
 void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 void count_launches(long long n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 long long launch_count() { return g_launches.load(std::memory_order_relaxed); }
+
+template cudaError_t launch_rhs_begin<float>(float *, const double *, long long, DevStatus *, cudaStream_t);
+template cudaError_t launch_rhs_begin<double>(double *, const double *, long long, DevStatus *, cudaStream_t);
+
+cudaError_t launch_factor_status(DevStatus *st, int mixed, cudaStream_t s)
+{
+    factor_status_kernel<<<1, 1, 0, s>>>(st, mixed);
+    count_launch();
+    return cudaGetLastError();
+}
 
 cudaError_t launch_relres(DevStatus *st, double tol, cudaStream_t s)
 {

@@ -621,44 +621,58 @@ __device__ __forceinline__ void tile_update_f32(float *sS, int o, int lane)
 // The lower tiles of sS are never read as matrix data (the Cholesky reads
 // the upper triangle), and (J, I) lies outside the diagonal tile being
 // factored while this runs.
-template <int LD, int PB>
+// A thread has COLS neighbouring columns of a row: with four, each scalar read
+// of V or T feeds four FMAs (one output per thread reads 5 words for 4 FMAs),
+// which takes a 128-wide chain step from 69 to 59 us; the 64-wide kernel, at
+// its 128 registers, spills with four and keeps one.
+template <int LD, int PB, int COLS>
 __device__ __forceinline__ void inv_column_par(float *sS, float *sV, int J, int t0, int nthr, int bar)
 {
-    const int total = J * PB * PB;
+    const int total = J * PB * PB / COLS;
     for (int e = t0; e < total; e += nthr) {
-        const int I = e / (PB * PB), w = e - I * PB * PB;
-        const int a = w % PB, c = w / PB;
-        float s0 = 0.f, s1 = 0.f;
+        const int I = e / (PB * PB / COLS), w = e - I * (PB * PB / COLS);
+        const int a = w % PB, c = COLS * (w / PB);
+        float s0[COLS] = {}, s1[COLS] = {};
         for (int P = I; P < J; ++P)
 #pragma unroll
             for (int q = 0; q < PB; q += 4) {
-                const float4 u = *reinterpret_cast<const float4 *>(sS + (PB * P + q) + (PB * J + c) * LD);  // U_PJ(q.., c)
-                const float *vr = sV + (PB * I + a) + (PB * P + q) * LD;                                   // V_IP(a, q..)
-                s0 = fmaf(vr[0], u.x, s0);
-                s1 = fmaf(vr[LD], u.y, s1);
-                s0 = fmaf(vr[2 * LD], u.z, s0);
-                s1 = fmaf(vr[3 * LD], u.w, s1);
+                const float *vr = sV + (PB * I + a) + (PB * P + q) * LD;  // V_IP(a, q..)
+                const float v0 = vr[0], v1 = vr[LD], v2 = vr[2 * LD], v3 = vr[3 * LD];
+#pragma unroll
+                for (int u4 = 0; u4 < COLS; ++u4) {
+                    const float4 u = *reinterpret_cast<const float4 *>(sS + (PB * P + q) + (PB * J + c + u4) * LD);  // U_PJ(q.., c)
+                    s0[u4] = fmaf(v0, u.x, s0[u4]);
+                    s1[u4] = fmaf(v1, u.y, s1[u4]);
+                    s0[u4] = fmaf(v2, u.z, s0[u4]);
+                    s1[u4] = fmaf(v3, u.w, s1[u4]);
+                }
             }
-        sS[(PB * J + a) + (PB * I + c) * LD] = s0 + s1;
+#pragma unroll
+        for (int u4 = 0; u4 < COLS; ++u4) sS[(PB * J + a) + (PB * I + c + u4) * LD] = s0[u4] + s1[u4];
     }
     if (bar == 0)
         __syncthreads();
     else
         asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(nthr) : "memory");
     for (int e = t0; e < total; e += nthr) {
-        const int I = e / (PB * PB), w = e - I * PB * PB;
-        const int a = w % PB, b = w / PB;
-        float s0 = 0.f, s1 = 0.f;
+        const int I = e / (PB * PB / COLS), w = e - I * (PB * PB / COLS);
+        const int a = w % PB, b = COLS * (w / PB);
+        float s0[COLS] = {}, s1[COLS] = {};
 #pragma unroll
         for (int c = 0; c < PB; c += 4) {
-            const float4 v = *reinterpret_cast<const float4 *>(sV + (PB * J + c) + (PB * J + b) * LD);  // V_JJ(c.., b)
-            const float *tr = sS + (PB * J + a) + (PB * I + c) * LD;                                   // T(a, c..)
-            s0 = fmaf(tr[0], v.x, s0);
-            s1 = fmaf(tr[LD], v.y, s1);
-            s0 = fmaf(tr[2 * LD], v.z, s0);
-            s1 = fmaf(tr[3 * LD], v.w, s1);
+            const float *tr = sS + (PB * J + a) + (PB * I + c) * LD;  // T(a, c..)
+            const float t0v = tr[0], t1v = tr[LD], t2v = tr[2 * LD], t3v = tr[3 * LD];
+#pragma unroll
+            for (int u4 = 0; u4 < COLS; ++u4) {
+                const float4 v = *reinterpret_cast<const float4 *>(sV + (PB * J + c) + (PB * J + b + u4) * LD);  // V_JJ(c.., b)
+                s0[u4] = fmaf(t0v, v.x, s0[u4]);
+                s1[u4] = fmaf(t1v, v.y, s1[u4]);
+                s0[u4] = fmaf(t2v, v.z, s0[u4]);
+                s1[u4] = fmaf(t3v, v.w, s1[u4]);
+            }
         }
-        sV[(PB * I + a) + (PB * J + b) * LD] = -(s0 + s1);
+#pragma unroll
+        for (int u4 = 0; u4 < COLS; ++u4) sV[(PB * I + a) + (PB * J + b + u4) * LD] = -(s0[u4] + s1[u4]);
     }
 }
 
@@ -725,10 +739,10 @@ __device__ __forceinline__ int chol_inv_blocked(T *sS, T *sV, T *dinv, int *sfla
                     if (bad && lane == 0) *sflag = 1;
                 } else {  // the rest of the trailing matrix, then V's block column K
                     trailing_update_f32<LD, NB, PB>(sS, o, PB, warp - 1, THREADS / 32 - 1, lane);
-                    if (K >= 1) inv_column_par<LD, PB>(sS, sV, K, tid - 32, THREADS - 32, 1);
+                    if (K >= 1) inv_column_par<LD, PB, NB >= 128 ? 4 : 1>(sS, sV, K, tid - 32, THREADS - 32, 1);
                 }
             } else if (K >= 1) {
-                inv_column_par<LD, PB>(sS, sV, K, tid, THREADS, 0);  // the last block column, all threads
+                inv_column_par<LD, PB, NB >= 128 ? 4 : 1>(sS, sV, K, tid, THREADS, 0);  // the last block column, all threads
             }
             __syncthreads();
         }
@@ -748,7 +762,7 @@ __device__ __forceinline__ int chol_inv_blocked(T *sS, T *sV, T *dinv, int *sfla
             if (bad && lane == 0) *sflag = 1;
         } else if (K >= 2) {
             if constexpr (FAST)
-                inv_column_par<LD, PB>(sS, sV, K - 1, tid - 32, THREADS - 32, 1);
+                inv_column_par<LD, PB, NB >= 128 ? 4 : 1>(sS, sV, K - 1, tid - 32, THREADS - 32, 1);
             else if constexpr (INL)
                 inv_column_i<T, LD, PB>(sS, sV, K - 1, tid - 32, THREADS - 32);
             else
@@ -783,7 +797,7 @@ __device__ __forceinline__ int chol_inv_blocked(T *sS, T *sV, T *dinv, int *sfla
     }
     if (KP > 1) {
         if constexpr (FAST)
-            inv_column_par<LD, PB>(sS, sV, KP - 1, tid, THREADS, 0);
+            inv_column_par<LD, PB, NB >= 128 ? 4 : 1>(sS, sV, KP - 1, tid, THREADS, 0);
         else if constexpr (INL)
             inv_column_i<T, LD, PB>(sS, sV, KP - 1, tid, THREADS);
         else

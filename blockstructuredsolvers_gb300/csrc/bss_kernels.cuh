@@ -92,10 +92,6 @@ template <>
 struct Tile<32> {
     static constexpr int TI = 16, TJ = 8, RA = 2, RB = 4, THREADS = 128;
 };
-template <>
-struct Tile<16> {
-    static constexpr int TI = 16, TJ = 4, RA = 1, RB = 4, THREADS = 64;
-};
 
 template <class T>
 struct Vec;
@@ -287,12 +283,6 @@ __device__ __forceinline__ void store_tile_smem(T *s, const T (&src)[Tile<NB>::R
     for (int a = 0; a < TL::RA; ++a)
 #pragma unroll
         for (int b = 0; b < TL::RB; ++b) s[(ti + TL::TI * a) + (tj + TL::TJ * b) * LD] = scale * src[a][b];
-}
-
-template <class T>
-__device__ __forceinline__ T safe_pivot(T p)
-{
-    return (p > T(0) && p < T(INFINITY)) ? p : T(1);
 }
 
 // ---------------------------------------------------------------------------

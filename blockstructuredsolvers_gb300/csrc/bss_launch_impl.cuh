@@ -62,7 +62,7 @@ static cudaError_t chain_factor_nb(const ChainFactorArgs<Tin, T> &a, cudaStream_
     if constexpr (std::is_same<T, float>::value && NB == 64) {
         if (!a.seq && !(a.variant & FACTOR_FMA_CHAIN)) return chain64_tc<Tin>(a, s);
     }
-    if constexpr (std::is_same<T, double>::value && NB >= 32) {
+    if constexpr (std::is_same<T, double>::value) {
         return chain_f64_tc<NB>(a, s);
     } else {
     const size_t smem = chain_factor_smem<T, NB>();
@@ -204,7 +204,7 @@ static int ctas_nb(int variant)
             return ctas_per_sm(kern, C64_THREADS, smem);
         }
     }
-    if constexpr (std::is_same<T, double>::value && NB >= 32) {
+    if constexpr (std::is_same<T, double>::value) {
         return NB == 64 ? 1 : 2;  // by shared memory and TMEM; by registers and TMEM
     }
     const size_t smem = chain_factor_smem<T, NB>();

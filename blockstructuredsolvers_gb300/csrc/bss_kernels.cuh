@@ -2732,7 +2732,7 @@ __device__ __forceinline__ void residual_rows_df(const double *__restrict__ Ag, 
     for (int q = 0; q < KB; ++q) sh[q] = sl[q] = 0.0f;
     float sa = 0.0f;
     if (has_b) {
-#pragma unroll 4
+#pragma unroll (KB > 4 ? 2 : 4)
         for (int c = c0; c < c1; ++c) {
             const float2 a = split_df(Ag[(long long)c * n]);
             const float2 b = split_df(Bg[(long long)c * n]);
@@ -2746,7 +2746,7 @@ __device__ __forceinline__ void residual_rows_df(const double *__restrict__ Ag, 
             }
         }
     } else {
-#pragma unroll 4
+#pragma unroll (KB > 4 ? 2 : 4)
         for (int c = c0; c < c1; ++c) {
             const float2 a = split_df(Ag[(long long)c * n]);
             if (NORM) sa += fabsf(a.x);
@@ -2760,6 +2760,32 @@ __device__ __forceinline__ void residual_rows_df(const double *__restrict__ Ag, 
 #pragma unroll
     for (int q = 0; q < KB; ++q) out[q * stride] = make_float2(sh[q], sl[q]);
     if (NORM) *rowsum = sa;
+}
+
+// u partials of RHS columns jb .. jb+KB-1: B_i(c0:c1, row)^T x_i from the
+// staged (split) column sB, each entry loaded once for the KB columns: one
+// column at a time took as many shared-memory cycles as FP32 ones (two
+// wavefronts and a broadcast per product).  With it and groups of eight
+// columns in the first phase (A_i and B_i split once, not per four columns)
+// k = 16 solves of N = 16384, n = 64 went 7570 -> 7204 us, N = 65536, n = 128,
+// k = 4 72.2 -> 70.9 ms, with the same sums in the same order.
+template <int KB>
+__device__ __forceinline__ void residual_cols_df(const float2 *sB, int c0, int c1, int n, const float2 *x0, float2 *out)
+{
+    float sh[KB], sl[KB];
+#pragma unroll
+    for (int q = 0; q < KB; ++q) sh[q] = sl[q] = 0.0f;
+#pragma unroll (KB > 1 ? 2 : 4)
+    for (int c = c0; c < c1; ++c) {
+        const float2 b = sB[c];
+#pragma unroll
+        for (int q = 0; q < KB; ++q) {
+            const float2 v = x0[c + q * n];
+            df_mac(b.x, b.y, v.x, v.y, sh[q], sl[q]);
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < KB; ++q) out[q * n] = make_float2(sh[q], sl[q]);
 }
 
 // column parts per block row for a CTA of THREADS threads (1 .. 8)
@@ -2935,12 +2961,19 @@ __device__ __forceinline__ void residual_body_df(const double *__restrict__ A, c
         if (active) {
             const double *Ag = (RAW ? rawA : A + i * nn) + row;
             const double *Bg = (RAW ? rawB : B + i * nn) + row;
-            // right-hand sides in compile-time groups (4, then 1); the first
-            // group also stages B_i and, when asked, the |A| + |B| row sums
+            // right-hand sides in compile-time groups (8, 4, then 1), each
+            // splitting A_i and B_i again; the first group also stages B_i
+            // and, when asked, the |A| + |B| row sums
             float *rs = rowred + part * n + row;
             float2 *o = red + part * k * n + row;
             int jb = 0;
-            if (k >= 4) {
+            if (k >= 8) {
+                if (with_norm)
+                    residual_rows_df<8, true>(Ag, Bg, has_b, c0, c1, n, LDp, x0, x1, sB + row, true, o, n, rs);
+                else
+                    residual_rows_df<8, false>(Ag, Bg, has_b, c0, c1, n, LDp, x0, x1, sB + row, true, o, n, rs);
+                jb = 8;
+            } else if (k >= 4) {
                 if (with_norm)
                     residual_rows_df<4, true>(Ag, Bg, has_b, c0, c1, n, LDp, x0, x1, sB + row, true, o, n, rs);
                 else
@@ -2966,14 +2999,11 @@ __device__ __forceinline__ void residual_body_df(const double *__restrict__ A, c
         }
         // phase 2: u_{i+1} partials from the staged B_i
         if (active && has_b) {
-            for (int j = 0; j < k; ++j) {
-                float sh = 0.0f, sl = 0.0f;
-                for (int c = c0; c < c1; ++c) {
-                    const float2 b = sB[c + row * LDp], v = x0[c + j * n];
-                    df_mac(b.x, b.y, v.x, v.y, sh, sl);
-                }
-                redu[(part * k + j) * n + row] = make_float2(sh, sl);
-            }
+            const float2 *bc = sB + row * LDp;
+            float2 *o = redu + part * k * n + row;
+            int jb = 0;
+            for (; jb + 4 <= k; jb += 4) residual_cols_df<4>(bc, c0, c1, n, x0 + jb * n, o + jb * n);
+            for (; jb < k; ++jb) residual_cols_df<1>(bc, c0, c1, n, x0 + jb * n, o + jb * n);
             if (with_norm) {
                 float sbt = 0.0f;
                 for (int c = c0; c < c1; ++c) sbt += fabsf(sB[c + row * LDp].x);

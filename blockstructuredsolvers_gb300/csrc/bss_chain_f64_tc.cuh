@@ -41,9 +41,10 @@
 // Measured (the digit products of one operand pair: 4.7K cycles for NB = 64,
 // 1.4K for NB = 32, against 131K and 16K for one product on the FP64 pipe):
 // plain FP64 factor + solve of N = 16384, n = 64: 35.6 -> 11.3 ms; N = 1531,
-// n = 37, k = 3: 6.42 -> 2.68 ms; N = 100, n = 32: 679 -> 435 us.  A 64-wide step
-// takes ~145K cycles: 49K in the four pivot tiles, 46K in the Cholesky's other
-// FP64 products, 31K cutting and putting together digits, 15K in MMAs.
+// n = 37, k = 3: 6.42 -> 2.68 ms; N = 100, n = 32: 679 -> 435 us (10.1 ms, 2.1 ms
+// and 378 us with the sweeps as they are now).  A 64-wide step takes ~145K cycles:
+// 49K in the four pivot tiles, 46K in the Cholesky's other FP64 products, 31K
+// cutting and putting together digits, 15K in MMAs.
 #pragma once
 
 namespace bss {

@@ -25,7 +25,8 @@ struct WlGeo {
     static constexpr uint32_t OFF_B = G::OFF_S;                               // two B operands
     static constexpr uint32_t B_BYTES = SL_DIGITS * G::VSLICE;
     static constexpr uint32_t OFF_EX = OFF_B + 2u * B_BYTES;                  // row exponents: slots 0, 1, B operands 0, 1
-    static constexpr uint32_t OFF_CTL = OFF_EX + 4u * 64u * 4u;
+    static constexpr uint32_t OFF_H = OFF_EX + 4u * 64u * 4u;                  // hV, hB of the block's 128 rows; none (64)
+    static constexpr uint32_t OFF_CTL = OFF_H + 5u * 64u * 4u;
     static constexpr uint32_t BYTES = OFF_CTL + 64u;
     static_assert(2 * G::TILE <= SL_DIGITS * G::SLICE, "sS and sV overlay the slots");
 };
@@ -36,6 +37,7 @@ struct WlTile {
     const double *p;  // the tile's first element; null: leave the operand alone
     int nk, nr;       // elements along K, operand rows (zero beyond)
     bool rows;
+    const int *h;     // the contraction index's balance (sl_balance)
 };
 
 __device__ __forceinline__ void wl_cut(unsigned char *dst, uint32_t group, uint32_t slice, int *exps, const WlTile &t,
@@ -43,7 +45,7 @@ __device__ __forceinline__ void wl_cut(unsigned char *dst, uint32_t group, uint3
 {
     const int r = 8 * gi + (threadIdx.x & 7);
     sl_cut_group<64>(dst + (uint32_t)gi * group, slice, exps + 8 * gi, t.p + (t.rows ? (long long)r : (long long)r * n),
-                     t.rows ? n : 1, r < t.nr ? t.nk : 0);
+                     t.rows ? n : 1, r < t.nr ? t.nk : 0, t.h);
 }
 
 // the accumulator, times sign, plus base, to a column tile of global memory:
@@ -99,6 +101,7 @@ __device__ __forceinline__ void chain128_f64_tc_body(const ChainFactorArgs<doubl
     unsigned char *OP = smem_sl, *OB = smem_sl + WlGeo::OFF_B;
     double *sS = reinterpret_cast<double *>(smem_sl), *sV = sS + Geo<double, 64>::SLOT;
     int *ex = reinterpret_cast<int *>(smem_sl + WlGeo::OFF_EX);
+    int *hV = reinterpret_cast<int *>(smem_sl + WlGeo::OFF_H), *hB = hV + 128, *hN = hB + 128;
     int *sflag = reinterpret_cast<int *>(smem_sl + WlGeo::OFF_CTL);
     const uint32_t aOP = smem_u32(OP), aOB = smem_u32(OB);
     const int tid = threadIdx.x, w = tid >> 5;
@@ -115,11 +118,11 @@ __device__ __forceinline__ void chain128_f64_tc_body(const ChainFactorArgs<doubl
         first = sL + 1;
         last = sR - 1;
     }
-    // tile (I, J) of a matrix
+    // tile (I, J) of a matrix; h: hV or hB where the contraction index is a row of the block
     auto at = [&](auto *M, int I, int J) { return M + 64 * I + (long long)64 * J * n; };
-    auto tile = [&](const double *M, int I, int J, bool rows = false) {
+    auto tile = [&](const double *M, int I, int J, bool rows = false, const int *h = nullptr) {
         const int a = I ? n1 : 64, b = J ? n1 : 64;
-        return WlTile{at(M, I, J), rows ? b : a, rows ? a : b, rows};
+        return WlTile{at(M, I, J), rows ? b : a, rows ? a : b, rows, h ? h + 64 * (rows ? J : I) : hN};
     };
     // cut x0, x1 into the slots and b0, b1 into the B operands (p null: left alone); ends with a barrier
     auto cut = [&](const WlTile &x0, const WlTile &x1, const WlTile &b0, const WlTile &b1) {
@@ -130,7 +133,7 @@ __device__ __forceinline__ void chain128_f64_tc_body(const ChainFactorArgs<doubl
         tc_fence_before();
         __syncthreads();
     };
-    const WlTile none{nullptr, 0, 0, false};
+    const WlTile none{nullptr, 0, 0, false, hN};
     // [slot 0 | slot 1]^T times operand b (0, 1: a slot; 2, 3: a B operand); false when the wait expired
     auto product = [&](int b) {
         if (tid == 0) {
@@ -171,6 +174,7 @@ __device__ __forceinline__ void chain128_f64_tc_body(const ChainFactorArgs<doubl
         __syncthreads();
     };
 
+    if (tid < 64) hN[tid] = -SL_BIAS;  // (read after factor's barriers)
     double *Cp = seq ? nullptr : g.C + p * 3 * nn;
     bool ok = true;
     for (long long i = first; i <= last && ok; ++i) {
@@ -200,32 +204,33 @@ __device__ __forceinline__ void chain128_f64_tc_body(const ChainFactorArgs<doubl
             __syncthreads();
         }
         // ---- blocked Cholesky and V_i = U^-1 in its slot
+        if (tid < 128) sl_balance(tid < n ? __ldcg(V + (long long)tid * (n + 1)) : 1.0, hV + tid, hB + tid);
         factor(V, 0, i);
-        cut(tile(V, 0, 0), none, tile(V, 0, 1), none);
+        cut(tile(V, 0, 0, false, hV), none, tile(V, 0, 1, false, hB), none);
         if (!(ok = emit(2, V, nullptr, nullptr, 1, true, false, 1.0))) break;  // U01 = V00^T S01
         cut(tile(V, 0, 1), none, tile(V, 0, 1), none);
         if (!(ok = product(2))) break;  // S11 -= U01^T U01
         wl_emit(cx.tm, ex, ex + 128, at(V, 1, 1), nullptr, at(V, 1, 1), nullptr, n1, 0, n1, n, -1.0);
         __syncthreads();
         factor(V, 1, i);
-        cut(tile(V, 0, 0, true), none, none, tile(V, 1, 1));  // (B operand 0 still holds U01)
+        cut(tile(V, 0, 0, true), none, none, tile(V, 1, 1, false, hV));  // (B operand 0 still holds U01)
         if (!(ok = emit(2, V, nullptr, nullptr, 1, true, false, 1.0))) break;  // T = V00 U01
-        cut(tile(V, 0, 1, true), none, none, none);
+        cut(tile(V, 0, 1, true, hB), none, none, none);
         if (!(ok = emit(3, V, nullptr, nullptr, 1, true, false, -1.0))) break;  // V01 = -T V11
         for (int e = tid; e < 64 * n1; e += SL_THREADS) at(V, 1, 0)[e % n1 + (long long)(e / n1) * n] = 0.0;
         // ---- Y_i = V^T Z, W_i = V^T B_i in place: the bottom row tiles of the inputs
         // first, then the top ones (rows of tile K are overwritten after they are cut;
         // the bottom tile of the result gets its second part with K = 0)
         for (int K = 1; K >= 0 && ok; --K) {
-            const WlTile x0 = K ? none : tile(V, 0, 0), x1 = tile(V, K, 1);
+            const WlTile x0 = K ? none : tile(V, 0, 0, false, hV), x1 = tile(V, K, 1, false, hV);
             if (!seq) {
-                cut(x0, x1, tile(Z, K, 0), tile(Z, K, 1));
+                cut(x0, x1, tile(Z, K, 0, false, hB), tile(Z, K, 1, false, hB));
                 for (int J = 0; J < 2 && ok; ++J) ok = emit(2 + J, Z, nullptr, K ? nullptr : Z, J, K == 0, true, 1.0);
             }
             if (has_next && ok) {
                 const double *B = g.B_in + i * nn;
                 double *W = g.B_f + i * nn;
-                cut(seq ? x0 : none, seq ? x1 : none, tile(B, K, 0), tile(B, K, 1));
+                cut(seq ? x0 : none, seq ? x1 : none, tile(B, K, 0, false, hB), tile(B, K, 1, false, hB));
                 for (int J = 0; J < 2 && ok; ++J) ok = emit(2 + J, W, nullptr, K ? nullptr : W, J, K == 0, true, 1.0);
             }
         }

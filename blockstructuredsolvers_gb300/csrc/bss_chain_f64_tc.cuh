@@ -15,9 +15,21 @@
 // the FP32 accumulator of the MMA.  Levels 0..7 (34 digit products; level 8 is
 // 2^-59 of the largest term) are put together in 64-bit integers and rounded
 // to FP64 once.  Error: the digits hold 54 bits below the power of two above
-// the row's largest element (a whole FP64 mantissa there), so a product of
-// random rows is off by ~2^-54 of the largest terms, against ~2^-53 for the
-// 64 roundings of an FP64 FMA chain.  Rows with an infinity or NaN give NaN.
+// the row's largest element, so a product is off by ~2^-54 of the product of
+// its two rows' largest elements.  That is an FP64 Cholesky's own error
+// (2^-53 sqrt(S_aa S_bb)) as long as the contraction index has one scale.  In
+// W^T W, Y^T W and Y^T Y it has: row r of W and Y is in units of the r-th
+// pivot's root.  In Z^T V and B^T V it has not: where T = D T0 D, row k of Z and
+// B goes with D_k and row k of V with 1 / D_k, and a row cut as it stands would
+// lose log2(max D / min D) bits.  There index k is first balanced by the power
+// of two h_k ~ sqrt(S_kk): 2^h_k V(k, .) and 2^-h_k Z(k, .), which cancel in the
+// product, are two operands of one scale (S balanced has diagonal [1, 4)); it
+// is an integer added to the exponents that the cut works with, and a result
+// does not depend on a D of powers of two at all.  D in 2^+-27, 19 blocks:
+// 2e-3 to 0.2 off without the balance, 1e-15 with it, at no cost (N = 16384,
+// n = 64: 10.10 -> 10.09 ms: S_LL and the cuts also moved between pivot tiles).  (An FMA chain also
+// keeps the small terms of a single balanced row; digits do not.)  Rows with an
+// infinity or NaN give NaN.
 //
 // A step of the chain (NB = 64 or 32, the block padded with the identity):
 //   P1 = [W_{i-1} | Y_{i-1}]^T W_{i-1}   -> S = A_i - W^T W (slot 0 rows), Z_i^T = -Y^T W (slot 1 rows)
@@ -62,8 +74,8 @@ struct SlGeo {
     static constexpr uint32_t OFF_S = SL_DIGITS * SLICE;         // sS; after the Cholesky sS and X hold the V operand
     static constexpr uint32_t OFF_X = OFF_S + TILE;              // Z in FP64; after P2 (sS, sX) hold W and Y in FP64
     static constexpr uint32_t OFF_V = OFF_X + TILE;              // sV
-    static constexpr uint32_t OFF_EX = OFF_V + TILE;             // row exponents: slot 0 (W, Z), Y, B (slot 1), V
-    static constexpr uint32_t OFF_CTL = OFF_EX + 4u * 64u * 4u;
+    static constexpr uint32_t OFF_EX = OFF_V + TILE;             // row exponents: slot 0 (W, Z), Y, B (slot 1), V; hV, hB, none
+    static constexpr uint32_t OFF_CTL = OFF_EX + 7u * 64u * 4u;
     static constexpr uint32_t BYTES = OFF_CTL + 64u;
     static constexpr uint32_t TMEM = SL_LEVELS * NB;
     static_assert(SL_DIGITS * VSLICE <= 2 * TILE, "the V operand overlays sS and X");
@@ -213,21 +225,30 @@ __device__ __forceinline__ void sl_read8(uint32_t addr, int er, const int *ec, d
     }
 }
 
-// the largest exponent field (at least 1) of a row as stored: the power of
-// two above the row's largest element
-__device__ __forceinline__ int sl_row_exp(int emax) { return emax == 2047 ? SL_NAN : emax - 1022; }
+// The balance of contraction index k: h_k, half the exponent of a diagonal
+// element of S (0 where it is no pivot), as what is added to the high words
+// of V's row k (hV) and of B's and Z's (hB): +-h_k in the exponent field's
+// place, less SL_BIAS, which keeps the sums of a field and h_k inside 32 bits.
+constexpr int SL_BIAS = 1 << 30;
+__device__ __forceinline__ void sl_balance(double s, int *hV, int *hB)
+{
+    const int E = __double2hiint(s) >> 20, h = (unsigned)E < 2047u ? (E - 1023) >> 1 : 0;
+    *hV = h * (1 << 20) - SL_BIAS;
+    *hB = -h * (1 << 20) - SL_BIAS;
+}
 
 // eight consecutive K values of one operand row as digits: 16 bytes per
-// digit at dst + s * stride.  emax: the row's largest exponent field.
-__device__ __forceinline__ void sl_put8(unsigned char *dst, uint32_t stride, const double (&x)[8], int emax)
+// digit at dst + s * stride.  fe: the values' exponent fields (at least 1) as
+// balanced, emax: the row's largest.
+__device__ __forceinline__ void sl_put8(unsigned char *dst, uint32_t stride, const double (&x)[8], const int (&fe)[8],
+                                        int emax)
 {
     uint32_t lo[8], hi[8];
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
         const unsigned xh = (unsigned)__double2hiint(x[q]), xl = (unsigned)__double2loint(x[q]);
-        const int E = (int)((xh >> 20) & 0x7FFu);
-        const unsigned mh = (xh & 0xFFFFFu) | (E ? 0x100000u : 0u);
-        int sh = emax - (E ? E : 1);
+        const unsigned mh = (xh & 0xFFFFFu) | ((xh & 0x7FF00000u) ? 0x100000u : 0u);
+        int sh = emax - fe[q];  // (negative only for a zero)
         // |x| 2^54 / 2^(row exponent), rounded: ((M << 2) >> sh) + 1 >> 1
         const unsigned h0 = __funnelshift_l(xl, mh, 2), l0 = xl << 2;
         const bool far = sh >= 32;
@@ -264,31 +285,66 @@ __device__ __forceinline__ void sl_put8(unsigned char *dst, uint32_t stride, con
 // one warp cuts eight operand rows into digits (lane: row lane % 8, quarter
 // lane / 8 of K) at dst (the row group's first core matrix of digit 0), their
 // exponents to exps[0..7].  row: the lane's row, its K values kstride apart,
-// zero from kvalid on.  Out of line: five callers, and the step's code should
-// stay in the instruction cache.
+// zero from kvalid on; value k is taken times 2^(+-h_k), h: hV or hB of
+// sl_balance (h_k = 0: -SL_BIAS).  Out of line, in one copy: five callers, and
+// the step's code should stay in the instruction cache.
 template <int NB>
 __device__ __noinline__ void sl_cut_group(unsigned char *dst, uint32_t stride, int *exps, const double *row,
-                                          long long kstride, int kvalid)
+                                          long long kstride, int kvalid, const int *h)
 {
     constexpr int KE = NB / 4;
     const int lane = threadIdx.x & 31, k0 = (lane >> 3) * KE;
     double x[KE];
-    int emax = 1 << 20;
+    int fe[KE];
+#pragma unroll
+    for (int q = 0; q < KE; ++q) x[q] = k0 + q < kvalid ? row[(k0 + q) * kstride] : 0.0;
+    // the row's largest high word (a field of at least 1) as balanced, zeros left out
+    constexpr int NAN_ROW = 0x7FFFFFFF;
+    int top = 0, emax = -NAN_ROW;
 #pragma unroll
     for (int q = 0; q < KE; ++q) {
-        x[q] = k0 + q < kvalid ? row[(k0 + q) * kstride] : 0.0;
-        emax = max(emax, __double2hiint(x[q]) & 0x7FFFFFFF);
+        const int mag = __double2hiint(x[q]) & 0x7FFFFFFF;
+        top = max(top, mag);
+        fe[q] = max(mag, 1 << 20) + h[k0 + q];
+        if ((mag | __double2loint(x[q])) != 0) emax = max(emax, fe[q]);
+        fe[q] >>= 20;
     }
+    if (top >= 0x7FF00000) emax = NAN_ROW;
     emax = max(emax, __shfl_xor_sync(0xFFFFFFFFu, emax, 8));
     emax = max(emax, __shfl_xor_sync(0xFFFFFFFFu, emax, 16));
+    if (lane < 8) exps[lane] = emax == NAN_ROW ? SL_NAN : (emax >> 20) + (SL_BIAS >> 20) - 1022;
     emax >>= 20;
-    if (lane < 8) exps[lane] = sl_row_exp(emax);
 #pragma unroll
     for (int q = 0; q < KE; q += 8) {
         const double x8[8] = {x[q], x[q + 1], x[q + 2], x[q + 3], x[q + 4], x[q + 5], x[q + 6], x[q + 7]};
-        sl_put8(dst + (uint32_t)((k0 + q) / 8) * 128u + (uint32_t)(lane & 7) * 16u, stride, x8, emax);
+        const int f8[8] = {fe[q], fe[q + 1], fe[q + 2], fe[q + 3], fe[q + 4], fe[q + 5], fe[q + 6], fe[q + 7]};
+        sl_put8(dst + (uint32_t)((k0 + q) / 8) * 128u + (uint32_t)(lane & 7) * 16u, stride, x8, f8, emax);
     }
     fence_async_smem();
+}
+
+// accumulator columns qa .. qb - 1 of this thread's row (m of a slot with row
+// exponents ex, columns the same slot's) to C, added where `add`; C null: none
+// of its own.  Out of line: three callers (see sl_cut_group).
+template <int NB>
+__device__ __noinline__ void sl_add(uint32_t tl, const int *ex, double *C, int m, int n, bool add, int qa, int qb)
+{
+    tc_fence_after();
+    const int er = ex[m];
+#pragma unroll 1
+    for (int q0 = qa; q0 < qb; q0 += 8) {
+        double v[8];
+        sl_read8<NB>(tl + (uint32_t)q0, er, ex + q0, v);
+        if (C) {
+            double c[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) c[q] = add && q0 + q < n ? __ldcg(C + (long long)(q0 + q) * n) : 0.0;
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+                if (q0 + q < n) __stcg(C + (long long)(q0 + q) * n, c[q] + v[q]);
+        }
+    }
+    tc_fence_before();
 }
 
 struct SlCtx {
@@ -310,6 +366,7 @@ __device__ __forceinline__ void chain_f64_tc_body(const ChainFactorArgs<double, 
     double *sV = reinterpret_cast<double *>(smem_sl + G::OFF_V);
     unsigned char *OV = smem_sl + G::OFF_S;                        // the V operand
     int *ex0 = reinterpret_cast<int *>(smem_sl + G::OFF_EX), *ex1 = ex0 + 64, *exB = ex1 + 64, *exV = exB + 64;
+    int *hV = exV + 64, *hB = hV + 64, *hN = hB + 64;
     int *sflag = reinterpret_cast<int *>(smem_sl + G::OFF_CTL);
     const uint32_t aOP = smem_u32(OP), aOV = smem_u32(OV);
 
@@ -334,6 +391,7 @@ __device__ __forceinline__ void chain_f64_tc_body(const ChainFactorArgs<double, 
     }
     double *Cp = seq ? nullptr : g.C + p * 3 * nn;
     for (int e = tid; e < Geo<double, NB>::SLOT; e += SL_THREADS) sV[e] = 0.0;  // V's strictly lower tiles stay zero
+    if (tid < NB) hN[tid] = -SL_BIAS;
     __syncthreads();
 
     // S_LL (+)= Y^T Y from the PL accumulator: its columns qa .. qb - 1, by warps 4-7
@@ -342,23 +400,7 @@ __device__ __forceinline__ void chain_f64_tc_body(const ChainFactorArgs<double, 
         asm volatile("bar.sync 3, 224;" ::: "memory");
     };
     auto add_sll = [&](bool add, int qa, int qb) {
-        if (*cx.abort || !live) return;
-        tc_fence_after();
-        const int er = ex1[m];
-#pragma unroll 1
-        for (int q0 = qa; q0 < qb; q0 += 8) {
-            double v[8];
-            sl_read8<NB>(tl + (uint32_t)q0, er, ex1 + q0, v);
-            if (slot == 1 && m < n) {
-                double c[8];
-#pragma unroll
-                for (int q = 0; q < 8; ++q) c[q] = add && q0 + q < n ? __ldcg(Cp + m + (long long)(q0 + q) * n) : 0.0;
-#pragma unroll
-                for (int q = 0; q < 8; ++q)
-                    if (q0 + q < n) __stcg(Cp + m + (long long)(q0 + q) * n, c[q] + v[q]);
-            }
-        }
-        tc_fence_before();
+        if (!*cx.abort && live) sl_add<NB>(tl, ex1, slot == 1 && m < n ? Cp + m : nullptr, m, n, add, qa, qb);
     };
     auto issue_pl = [&]() {
         if (tid == 128) {  // (not warp 0: an MMA holds its issuing thread for its duration)
@@ -428,24 +470,34 @@ __device__ __forceinline__ void chain_f64_tc_body(const ChainFactorArgs<double, 
             __syncthreads();
             if (!seq) issue_pl();
         }
-        // ---- Cholesky + inverse; beside the first two pivot tiles S_LL (warps 4-7) and
-        // the digits of B_i (slot 1) and Z_i (slot 0; first block: B_sL^T) (warps 1-3)
+        // ---- Cholesky + inverse; beside the pivot tiles S_LL (warps 4-7) and the digits of
+        // B_i (slot 1) and Z_i (slot 0; first block: B_sL^T) (warps 1-3).  A 64-wide block's
+        // are spread so that they end with the pivot tile they run beside (14K cycles, 4K of the
+        // first one's spent waiting for PL; 8 columns of S_LL take 3K, a group of 8 rows 3K to 5K).
         auto aside = [&](int K) {
             const bool pl = t > 0 && !seq;
-            if (K == 0 && pl) wait_pl();
-            if (K <= 1 && w >= 4) {
-                constexpr int PART = (5 * NB / 8 + 7) / 8 * 8;  // most of them beside the first, which starts late
-                if (pl) add_sll(t > 1, K == 0 ? 0 : PART, K == 0 ? PART : NB);
-            } else if (K <= 1) {
-                for (int gi = w - 1; gi < NB / 8; gi += 3) {
-                    const int row = 8 * gi + (lane & 7), valid = row < n ? n : 0;
-                    unsigned char *dst = OP + (uint32_t)(2 * gi + 1 - K) * G::GRP;
-                    if (K == 0 && has_next)
-                        sl_cut_group<NB>(dst, G::SLICE, exB + 8 * gi, g.B_in + i * nn + (long long)row * n, 1, valid);
-                    else if (K == 1 && pl)
-                        sl_cut_group<NB>(dst, G::SLICE, ex0 + 8 * gi, sX + row * LD, 1, NB);
-                    else if (K == 1 && !seq)
-                        sl_cut_group<NB>(dst, G::SLICE, ex0 + 8 * gi, g.B_in + sL * nn + row, n, valid);
+            if (K == 0) {  // the balance of B_i, Z_i and V_i, before the pivots change S's diagonal
+                if (w <= 3 && tid - 32 < NB) sl_balance(sS[(tid - 32) * (LD + 1)], hV + tid - 32, hB + tid - 32);
+                if (pl) wait_pl();
+                else if (w <= 3) asm volatile("bar.sync 4, 96;" ::: "memory");
+            }
+            constexpr int NG = NB / 8;
+            constexpr int S1 = 24, S2 = NB == 64 ? 56 : NB;                // columns of S_LL
+            constexpr int B1 = NB == 64 ? 6 : NG, B2 = NB == 64 ? 7 : NG;  // row groups of B_i
+            if (w >= 4) {
+                const int qa = K == 0 ? 0 : K == 1 ? S1 : S2, qb = K == 0 ? S1 : K == 1 ? S2 : K == 2 ? NB : S2;
+                if (pl && qa < qb) add_sll(t > 1, qa, qb);
+            } else {
+                const int ua = K == 0 ? 0 : !pl ? NG : K == 1 ? B1 : K == 2 ? B2 : NG;
+                const int ub = !pl ? NG : K == 0 ? B1 : K == 1 ? B2 : NG;
+                for (int u = ua + w - 1; u < ub + (K == 1 ? NG : 0); u += 3) {
+                    const bool isB = u < ub;
+                    if (isB ? !has_next : seq) continue;
+                    const int gi = isB ? u : u - ub, r = 8 * gi + (lane & 7);
+                    const double *row = isB ? g.B_in + i * nn + (long long)r * n : pl ? sX + r * LD : g.B_in + sL * nn + r;
+                    sl_cut_group<NB>(OP + (uint32_t)(2 * gi + (isB ? 1 : 0)) * G::GRP, G::SLICE,
+                                           (isB ? exB : ex0) + 8 * gi, row, isB || pl ? 1 : n,
+                                           !isB && pl ? NB : r < n ? n : 0, hB);
                 }
             }
         };
@@ -454,7 +506,7 @@ __device__ __forceinline__ void chain_f64_tc_body(const ChainFactorArgs<double, 
         if (*cx.abort) break;
         // ---- V_i's digits over sS and sX, V_i to global memory while P2 = [Z_i | B_i]^T V_i runs
         if (has_next) {
-            if (w < NB / 8) sl_cut_group<NB>(OV + (uint32_t)w * G::GRP, G::VSLICE, exV + 8 * w, sV + (8 * w + (lane & 7)) * LD, 1, NB);
+            if (w < NB / 8) sl_cut_group<NB>(OV + (uint32_t)w * G::GRP, G::VSLICE, exV + 8 * w, sV + (8 * w + (lane & 7)) * LD, 1, NB, hV);
             tc_fence_before();
             __syncthreads();
             if (tid == 0) {
@@ -496,9 +548,9 @@ __device__ __forceinline__ void chain_f64_tc_body(const ChainFactorArgs<double, 
             const int gi = u >> 1, row = 8 * gi + (lane & 7);
             unsigned char *dst = OP + (uint32_t)(2 * gi + (u & 1)) * G::GRP;
             if (u & 1) {
-                if (!seq) sl_cut_group<NB>(dst, G::SLICE, ex1 + 8 * gi, sX + row * LD, 1, NB);
+                if (!seq) sl_cut_group<NB>(dst, G::SLICE, ex1 + 8 * gi, sX + row * LD, 1, NB, hN);
             } else {
-                sl_cut_group<NB>(dst, G::SLICE, ex0 + 8 * gi, sS + row * LD, 1, NB);
+                sl_cut_group<NB>(dst, G::SLICE, ex0 + 8 * gi, sS + row * LD, 1, NB, hN);
             }
         }
         __syncthreads();

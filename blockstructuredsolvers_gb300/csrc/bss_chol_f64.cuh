@@ -261,7 +261,7 @@ __device__ __forceinline__ constexpr int f64_aside()
 }
 
 // `aside(K)` runs on the warps other than warp 0 while that factors pivot tile
-// K: the caller's own work, which must not touch sS or sV.
+// K: the caller's own work, which must not write sS or sV.
 struct F64NoAside {
     __device__ __forceinline__ void operator()(int) const {}
 };

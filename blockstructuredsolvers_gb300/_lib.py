@@ -47,7 +47,7 @@ EXPORTS = (
     "bss_server_release", "bss_server_get_stats", "bss_server_reset_stats",
     "bss_autotune", "bss_autotune_lookup", "bss_autotune_clear", "bss_autotune_save", "bss_autotune_load",
     "bss_cpu_create", "bss_cpu_destroy", "bss_cpu_get_tensors", "bss_cpu_factorize", "bss_cpu_solve",
-    "bss_cpu_failed_block", "bss_tc_selftest", "bss_diag_wide_occupancy", "bss_diag_residual",
+    "bss_cpu_failed_block", "bss_tc_selftest", "bss_diag_pivot_selftest", "bss_diag_wide_occupancy", "bss_diag_residual",
     "bss_diag_wait_timeout", "bss_diag_fma_peak", "bss_diag_set_factor_variant", "bss_diag_get_factor_variant",
     "bss_refalgo_create", "bss_refalgo_destroy", "bss_refalgo_get_tensors", "bss_refalgo_get_dims",
     "bss_refalgo_factorize", "bss_refalgo_solve",
@@ -222,6 +222,7 @@ def load(path: str | None = None):
     L.bss_cpu_solve.argtypes = [vp]
     L.bss_cpu_failed_block.argtypes = [vp, ctypes.POINTER(i64)]
     L.bss_tc_selftest.argtypes = [i64, ctypes.POINTER(ctypes.c_double)]
+    L.bss_diag_pivot_selftest.argtypes = [ctypes.POINTER(ctypes.c_int32)] * 2
     L.bss_diag_wide_occupancy.argtypes = [ctypes.POINTER(i64)]
     L.bss_diag_residual.argtypes = [i64, i64, i64, i32, vp, vp, vp, vp, vp, vp]
     L.bss_diag_wait_timeout.argtypes = [i64, ctypes.POINTER(i64), ctypes.POINTER(i64)]

@@ -181,6 +181,53 @@ extern "C" int bss_diag_wait_timeout(int64_t polls, int64_t *timed_out, int64_t 
     return BSS_OK;
 }
 
+namespace {
+__device__ int ulps_apart(double a, double b)
+{
+    const long long d = __double_as_longlong(a) - __double_as_longlong(b);
+    return (int)min(d < 0 ? -d : d, 0x7FFFFFFFll);
+}
+
+// Both are functions of a pivot's upper 23 mantissa bits (the FP32 seed), its
+// lower 29 and its exponent: every seed, the lower bits all zero and all one,
+// exponents of both parities and the ends of the ordinary range.
+__global__ void diag_pivot_kernel(int *worst)
+{
+    int rcp = 0, rsqrt = 0;
+    const int step = gridDim.x * blockDim.x;
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < 1 << 24; e += step) {
+        const long long frac = ((long long)(e >> 1) << 29) | ((e & 1) ? (1ll << 29) - 1 : 0ll);
+        for (int q = 0; q < 4; ++q) {
+            const long long ex = q == 0 ? 24 : q == 1 ? 1023 : q == 2 ? 1024 : 2022;
+            const double p = __longlong_as_double((ex << 52) | frac);
+            rcp = max(rcp, ulps_apart(f64_rcp(p), 1.0 / p));
+            rsqrt = max(rsqrt, ulps_apart(f64_rsqrt(p), 1.0 / sqrt(p)));
+        }
+    }
+    atomicMax(worst, rcp);
+    atomicMax(worst + 1, rsqrt);
+}
+}  // namespace
+
+extern "C" int bss_diag_pivot_selftest(int32_t *rcp_ulps, int32_t *rsqrt_ulps)
+{
+    if (!rcp_ulps || !rsqrt_ulps) return fail(BSS_ERR_ARG, "bss_diag_pivot_selftest: output is NULL");
+    int *d = nullptr, h[2] = {0, 0};
+    BSS_CUDA(cudaMalloc((void **)&d, sizeof(h)));
+    cudaError_t e = cudaMemset(d, 0, sizeof(h));
+    if (e == cudaSuccess) {
+        diag_pivot_kernel<<<1024, 256>>>(d);
+        count_launch();
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(h, d, sizeof(h), cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    if (e != cudaSuccess) return cuda_fail(e, "bss_diag_pivot_selftest");
+    *rcp_ulps = h[0];
+    *rsqrt_ulps = h[1];
+    return BSS_OK;
+}
+
 // ---------------------------------------------------------------------------
 // FMA-pipe peak microbenchmark: every thread runs 8 independent FMA chains
 // (enough to cover the pipe latency with 8 warps per scheduler) for `iters`

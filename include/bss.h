@@ -467,6 +467,12 @@ int bss_diag_wait_timeout(int64_t polls, int64_t *timed_out, int64_t *cycles);
  * compute peak of the FP32 and FP64 paths.  Synchronises the device. */
 int bss_diag_fma_peak(int32_t dtype, double *tflops);
 
+/* Diagnostic (no counterpart in the reference): the FP64 Cholesky's pivot
+ * reciprocal and reciprocal square root, which start from an FP32 seed, over
+ * every seed mantissa: the largest difference, in units of the last place,
+ * from 1 / p and 1 / sqrt(p).  Synchronises the device. */
+int bss_diag_pivot_selftest(int32_t *rcp_ulps, int32_t *rsqrt_ulps);
+
 /* Kernel variants of the chain factorization (bits; no counterpart in the
  * reference).  BSS_FACTOR_FMA_CHAIN: partitioned levels of 33 <= n <= 64
  * blocks with FP32 factors (plain FP32, and every level of the mixed path)

@@ -288,8 +288,16 @@ template <class Tin, class T>
 void plan_factor_level(Builder &B, int level, bool coarsest)
 {
     bss_batch *b = B.b;
-    // wide blocks: the tensor-core form (FP32, n <= 128) is its own launch class
-    for (int nb : {16, 32, 64, (int)WIDE_CLASS, (int)WIDE_CLASS + 1}) {
+    // wide blocks: the tensor-core form (FP32, n <= 128) is its own launch class;
+    // partitioned FP32 levels whose variant asks for the kernel without the
+    // on-chip chain step (FACTOR_*) are another
+    struct Class {
+        int nb;
+        bool alt;
+    };
+    for (const Class cl : {Class{16, false}, Class{32, false}, Class{64, false}, Class{64, true}, Class{WIDE_CLASS, false},
+                           Class{WIDE_CLASS + 1, false}, Class{WIDE_CLASS + 1, true}}) {
+        const int nb = cl.nb;
         std::vector<ChainFactorArgs<Tin, T>> descs;
         std::vector<WorkItem> items;
         std::vector<long long> len;
@@ -299,7 +307,9 @@ void plan_factor_level(Builder &B, int level, bool coarsest)
             const int l = coarsest ? L - 1 : level;
             int cls = nb_class(h->n);
             if (cls == WIDE_CLASS && wide_uses_tc<T>((int)h->n)) cls = WIDE_CLASS + 1;
-            if (cls != nb || l >= L) continue;
+            const int bit = cls == 64 ? FACTOR_FMA_CHAIN : cls == WIDE_CLASS + 1 ? FACTOR_WIDE_L2 : 0;
+            const bool alt = std::is_same<T, float>::value && !coarsest && (h->variant & bit) != 0;
+            if (cls != nb || alt != cl.alt || l >= L) continue;
             const Level &lv = h->levels[l];
             if (lv.seq != coarsest) continue;
             if ((lv.tin == F64) != std::is_same<Tin, double>::value || (lv.t == F64) != std::is_same<T, double>::value)
@@ -324,7 +334,7 @@ void plan_factor_level(Builder &B, int level, bool coarsest)
         size_t om = 0;
         bool tma = true;
         if constexpr (std::is_same<T, float>::value) {
-            if (nb == WIDE_CLASS + 1 && !coarsest) {
+            if (nb == WIDE_CLASS + 1 && !coarsest && !cl.alt) {
                 std::vector<CUtensorMap> maps(descs.size());
                 for (size_t q = 0; q < descs.size(); ++q)
                     tma = (chain128_tmap_b<Tin>(descs[q], &maps[q]) || descs[q].n % 2 != 0) && tma;  // (odd n: plain loads)
@@ -336,10 +346,10 @@ void plan_factor_level(Builder &B, int level, bool coarsest)
             st.what = std::string("plan_factor_level") + " items=" + std::to_string(ni);
             st.run = [=](cudaStream_t s) {
                 if constexpr (std::is_same<T, float>::value) {
-                    if (nb == 64 && !coarsest)
+                    if (nb == 64 && !coarsest && !cl.alt)
                         return queue_factor64_tc<Tin>((const ChainFactorArgs<Tin, T> *)(base + od),
                                                       (const WorkItem *)(base + oi), ni, (int *)(base + oh), sms, s);
-                    if (nb == WIDE_CLASS + 1 && !coarsest)
+                    if (nb == WIDE_CLASS + 1 && !coarsest && !cl.alt)
                         return queue_factor128_tc<Tin>((const ChainFactorArgs<Tin, T> *)(base + od),
                                                        (const CUtensorMap *)(base + om), tma,
                                                        (const WorkItem *)(base + oi), ni, (int *)(base + oh), sms, s);

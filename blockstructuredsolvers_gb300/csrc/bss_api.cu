@@ -385,7 +385,7 @@ int create_common(bss_handle *h, int64_t N, int64_t n, int64_t k, int32_t dtype,
     // columns per pass by the type of the sweeps' levels: FP32 in mixed precision,
     // unless its coarsest level stays FP64
     const bool f32 = h->opt.precision == BSS_PRECISION_MIXED && !h->opt.coarsest_fp64;
-    h->kc_max = solve_kc_max((int)n, (int)k, f32 ? 4 : (int)tsize(dtype));
+    h->kc_max = solve_columns((int)n, (int)k, f32 ? 4 : (int)tsize(dtype));
     int rc = build_handle(h);
     if (rc != BSS_OK) {
         if (h->arena) cudaFree(h->arena);

@@ -72,7 +72,11 @@ cudaError_t launch_update(double *x, const Tc *c, long long count, int assign, c
 template <class T>
 cudaError_t launch_init_identity(T *A, long long first_blk, long long last_blk, int n, cudaStream_t s);
 
+// most columns of one pass in the form that one column takes
 int solve_kc_max(int n, int k, int elem_bytes);
+// columns per pass of a handle that may take several (a batch and the
+// no-allocation call keep solve_kc_max: what they refuse depends on it)
+int solve_columns(int n, int k, int elem_bytes);
 
 // resident CTAs per SM of a kernel: the larger of the occupancy query and
 // the count from its registers and shared memory (the query reports one CTA

@@ -298,7 +298,7 @@ Factor *plan_factor(bss_server *S, Request *r)
     h->k = r->k;
     h->dtype = F64;
     h->device = S->device;
-    h->kc_max = solve_kc_max((int)r->n, (int)r->k, h->opt.precision == BSS_PRECISION_MIXED && !h->opt.coarsest_fp64 ? 4 : 8);
+    h->kc_max = solve_columns((int)r->n, (int)r->k, h->opt.precision == BSS_PRECISION_MIXED && !h->opt.coarsest_fp64 ? 4 : 8);
     plan_handle(h);
     h->arena_bytes = (h->arena_bytes + 255) & ~(size_t)255;
     Factor *f = new Factor();

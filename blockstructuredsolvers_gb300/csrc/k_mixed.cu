@@ -81,4 +81,24 @@ int solve_kc_max(int n, int k, int elem_bytes)
     }
     return best;
 }
+
+int solve_columns(int n, int k, int elem_bytes)
+{
+    // A staged pass of eight columns or more beats the unstaged forms even where
+    // it takes more passes; one of fewer does not (mixed solve, N ~ 2800: n = 92,
+    // k = 32, four staged passes 8.0 ms, one unstaged 10.0; n = 94, k = 16, four of
+    // five columns 6.3 ms, one unstaged 5.2; n = 96, k = 8, one column at a time
+    // 4.1 ms, streamed 2.4).  That is FP32 with n = 93..96.
+    const int staged = solve_kc_max(n, k, elem_bytes);
+    if (staged >= 8 || staged >= k) return staged;
+    int best = 1;
+    for (int kc = 1; kc <= 32 && kc <= k; ++kc) {
+        const size_t need = elem_bytes == 8 ? solve_smem_bytes<double>(n, kc, false) : solve_smem_bytes<float>(n, kc, false);
+        if (need > SOLVE_SMEM_MAX) break;
+        best = kc;
+    }
+    // the streamed sweeps, where they serve, take eight (k = 12: 8 + 4 columns 3.9 ms, 12 direct 4.4)
+    if (best > 8 && (elem_bytes == 8 ? solve_streamed<double>(n, 8) : solve_streamed<float>(n, 8))) best = 8;
+    return best;
+}
 }  // namespace bss

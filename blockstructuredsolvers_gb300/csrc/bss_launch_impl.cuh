@@ -288,14 +288,35 @@ static cudaError_t launch_chained(void (*kern)(P...), unsigned grid, int threads
     return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
+static int device_sms()
+{
+    int dev = 0, sms = 1;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
+}
+
 template <class T>
 static int sweep_threads(const SolveArgs<T> &a, bool staged)
 {
     if (!staged || a.seq) return SOLVE_THREADS;
-    int dev = 0, sms = 1;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return solve_threads(a.n, a.kc, a.Q, sms);
+    return solve_threads(a.n, a.kc, a.Q, device_sms());
+}
+
+// Whether a sweep starts under the one before it (see pdl_release_next), the
+// larger of the two levels having `partitions`.  It gains the launch and the
+// first loads, 2 to 3 us a level.  But CTAs that start early go where there is
+// room, two to an SM where two fit, and stay there; when the earlier level
+// fills the SMs that doubles a step's time.  Unstaged steps are long, and
+// several CTAs always fit.  Solve, all levels chained / by this rule / none,
+// separate launches in stream order with assembled right-hand sides = 1: FP64 N = 4000 n = 20 k = 16 1.41 / 0.81 /
+// 0.71, N = 964 n = 72 k = 1 1.14 / 1.01 / 1.01; N = 4000 n = 16 k = 1 0.52 / 0.48 /
+// 0.53, FP32 n = 40 k = 16 1.14 / 0.97 / 1.01, n = 16 k = 1 0.62 / 0.61 / 0.71,
+// N = 33 n = 32 k = 1 (few partitions) FP64 0.56 / 0.55 / 0.66, FP32 0.70 / 0.69 / 0.89.
+static bool chains(bool staged, size_t smem, long long partitions)
+{
+    const bool two_fit = 2 * smem <= 227 * 1024;
+    return staged && !(two_fit && 2 * partitions > device_sms());
 }
 
 template <class T>
@@ -323,7 +344,7 @@ cudaError_t launch_chain_fwd(const SolveArgs<T> &a, cudaStream_t s)
     cudaError_t e = set_solve_smem<T>((const void *)kern, smem);
     if (e != cudaSuccess) return e;
     const unsigned grid = a.seq ? 1u : (unsigned)a.Q;
-    if (a.chained) e = launch_chained(kern, grid, sweep_threads<T>(a, staged), smem, s, a);
+    if (a.chained && chains(staged, smem, a.fine_Q)) e = launch_chained(kern, grid, sweep_threads<T>(a, staged), smem, s, a);
     else kern<<<grid, sweep_threads<T>(a, staged), smem, s>>>(a);
     count_launch();
     return e != cudaSuccess ? e : cudaGetLastError();
@@ -346,7 +367,7 @@ cudaError_t launch_chain_bwd(const SolveArgs<T> &a, cudaStream_t s)
     auto kern = staged ? chain_bwd_kernel<T, Tsep, true> : chain_bwd_kernel<T, Tsep, false>;
     cudaError_t e = set_solve_smem<T>((const void *)kern, smem);
     if (e != cudaSuccess) return e;
-    if (a.chained) e = launch_chained(kern, (unsigned)a.Q, sweep_threads<T>(a, staged), smem, s, a);
+    if (a.chained && chains(staged, smem, a.Q)) e = launch_chained(kern, (unsigned)a.Q, sweep_threads<T>(a, staged), smem, s, a);
     else kern<<<(unsigned)a.Q, sweep_threads<T>(a, staged), smem, s>>>(a);
     count_launch();
     return e != cudaSuccess ? e : cudaGetLastError();

@@ -2043,7 +2043,7 @@ __device__ __forceinline__ void store_rhs(Tg *__restrict__ g, const T *s, long l
 
 // x - l - r rounded once: FP32 by error-free differences (Knuth's TwoSum),
 // whose FP32 instructions are far cheaper here than three conversions to FP64;
-// in FP64 where a difference leaves the FP32 range (an infinity makes the
+// in halves where a difference leaves the FP32 range (an infinity makes the
 // error terms NaN), although the result may not
 __device__ __forceinline__ double minus_both(double x, double l, double r) { return x - l - r; }
 __device__ __forceinline__ float minus_both(float x, float l, float r)
@@ -2053,7 +2053,7 @@ __device__ __forceinline__ float minus_both(float x, float l, float r)
     const float t = __fsub_rn(s, r), tb = __fsub_rn(t, s);
     const float et = __fsub_rn(__fsub_rn(s, __fsub_rn(t, tb)), __fadd_rn(r, tb));
     const float y = __fadd_rn(t, __fadd_rn(es, et));
-    return isfinite(y) ? y : (float)((double)x - (double)l - (double)r);
+    return isfinite(y) ? y : 2.f * (0.5f * x - 0.5f * l - 0.5f * r);
 }
 
 // block s of a coarser level's RHS, from the finer level's: d'_s = d_{sep s} -

@@ -1519,11 +1519,24 @@ struct TmulOp {
     bool minus, add;
 };
 
+// Chunks by which the walk of column c + 1 starts ahead of column c's: a
+// wavefront reads eight columns' chunks of `shares` neighbouring shares (one
+// for 16-byte chunks, two, four), which meet no bank twice when a column's
+// length and this turn add up to an odd number of `shares`.  (Always one chunk,
+// eight columns of 28, 60 or 92 floats met in one bank: forward and backward
+// sequential sweep of 33 blocks, n = 94, 190 -> 225 us against the form before.)
+template <class T, int W>
+__device__ __forceinline__ int tmul_turn(int nch)
+{
+    constexpr int shares = 16 / (W * (int)sizeof(T));
+    return (shares - nch) & (2 * shares - 1);
+}
+
 // One or two such products with the same v (two to four right-hand sides at a
 // time).  A warp takes 8 CT columns x JT
 // right-hand sides: lane = column (lane % 8), share of the contraction (lane
 // / 8, every fourth chunk of W rows), the shares added by shuffles.  Each
-// lane starts its walk lane % 8 chunks in, so that the eight columns of an
+// column's walk starts some chunks in (tmul_turn), so that the columns of an
 // access fall into distinct banks of the unpadded block.  tri: M upper
 // triangular, chunks wholly below the warp's columns are skipped.
 // What bounds it: in FP64 the FP64 pipe, whose instructions cost the same for
@@ -1539,7 +1552,7 @@ __device__ __noinline__ void cta_tmul_t(const TmulOp a, const TmulOp b, int nops
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T *sm = reinterpret_cast<T *>(smem_raw);
     const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    const int j8 = lane & 7, part = lane >> 3, nch = n / W;
+    const int j8 = lane & 7, part = lane >> 3, nch = n / W, turn = tmul_turn<T, W>(nch);
     const int G = (n + 8 * CT - 1) / (8 * CT), JG = (kc + JT - 1) / JT;
     // this warp's tasks: every nw-th of (operation, right-hand-side group, column group)
     int cg = threadIdx.x >> 5, jg = 0;
@@ -1567,7 +1580,7 @@ __device__ __noinline__ void cta_tmul_t(const TmulOp a, const TmulOp b, int nops
         T acc[JP * CT];  // (j, t), j padded to a power of two
 #pragma unroll
         for (int i = 0; i < JP * CT; ++i) acc[i] = T(0);
-        int ch = part + j8;
+        int ch = part + j8 * turn;
         while (ch >= lim) ch -= lim;
 #pragma unroll 2
         for (int q = part; q < lim; q += 4) {
@@ -1841,7 +1854,7 @@ __device__ __forceinline__ void cta_tmul_1(const TmulOp a, const TmulOp b, int n
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T *sm = reinterpret_cast<T *>(smem_raw);
     const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    const int j8 = lane & 7, part = lane >> 3, nch = n / W, G = (n + 7) >> 3;
+    const int j8 = lane & 7, part = lane >> 3, nch = n / W, turn = tmul_turn<T, W>(nch), G = (n + 7) >> 3;
     const T *v = sm + v0;
     for (int u = threadIdx.x >> 5; u < nops * G; u += nw) {
         const bool second = u >= G;
@@ -1849,7 +1862,7 @@ __device__ __forceinline__ void cta_tmul_1(const TmulOp a, const TmulOp b, int n
         const int lim = tri ? min(nch, (c8 + 8 + W - 1) / W) : nch;
         const T *m = sm + (second ? b.M : a.M) + min(c, n - 1) * n;
         T acc = T(0);
-        int ch = part + j8;
+        int ch = part + j8 * turn;
         while (ch >= lim) ch -= lim;
 #pragma unroll 4
         for (int q = part; q < lim; q += 4) {

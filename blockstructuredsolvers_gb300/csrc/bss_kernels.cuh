@@ -1880,6 +1880,61 @@ __device__ __forceinline__ void cta_tmul_1(const TmulOp a, const TmulOp b, int n
     }
 }
 
+// Whole outputs per thread: thread = (column c, the right-hand sides jg,
+// jg + tpc, ... with tpc = threads / n), the lanes starting their walks at
+// different offsets so that they hit distinct banks; n even.
+static __device__ __noinline__ void cta_tmul_s(const TmulOp a, const TmulOp b, int nops, int v0, int n, int kc)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double *sm = reinterpret_cast<double *>(smem_raw);
+    const int tpc = (int)blockDim.x / n;
+    const int c = threadIdx.x % n, jg = threadIdx.x / n;
+    if (jg >= tpc) return;
+    const int rot = (2 * (threadIdx.x & 7)) % n;
+    const double *v = sm + v0;
+    for (int p = 0; p < nops; ++p) {
+        const TmulOp &o = p ? b : a;
+        const double *mc = sm + o.M + c * n;
+        double *out = sm + o.out + c;
+        for (int j0 = jg; j0 < kc; j0 += 4 * tpc) {
+            double acc[4] = {0.0, 0.0, 0.0, 0.0};
+            for (int r2 = 0; r2 < n; r2 += 2) {
+                int r = r2 + rot;
+                if (r >= n) r -= n;
+                const double2 m = *reinterpret_cast<const double2 *>(mc + r);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int j = j0 + tpc * q;
+                    if (j < kc) fma_vec(acc[q], m, *reinterpret_cast<const double2 *>(v + r + j * n));
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int j = j0 + tpc * q;
+                if (j < kc) {
+                    const double x = o.minus ? -acc[q] : acc[q];
+                    out[j * n] = o.add ? out[j * n] + x : x;
+                }
+            }
+        }
+    }
+}
+
+// FP64 with many right-hand sides, where the split form above issues more
+// FP64 instructions: blocks of a few columns, mostly padding of its eight
+// columns x four shares, and right-hand sides that fill the four of a thread
+// here.  (Solve of N = 4000 with this / the split form, the ordered launches of
+// assembled right-hand sides = 1: n = 2 k = 32 1.02 / 1.63, n = 10 k = 32 1.12 / 1.24,
+// n = 42 k = 24 1.02 / 1.22, n = 58 k = 16 1.02 / 1.10; n = 48 k = 16, three of the four
+// filled, 1.02 / 0.86.)
+__device__ __forceinline__ bool tmul_whole(int n, int kc)
+{
+    if (kc < 12 || n % 2 != 0 || n > (int)blockDim.x) return false;
+    const int padded = ((n + 7) & ~7) * ((n + 7) & ~7);
+    return n <= 4 || (padded > 2 * n * n && kc > 24) ||
+           (n * kc > 3 * (int)blockDim.x && (kc + 3) / 4 * n <= (int)blockDim.x);
+}
+
 // Transpose products of blocks staged in shared memory: W = the widest vector
 // that every column starts on; with many right-hand sides in FP32 a warp takes
 // 2 or 4 column groups at once, as long as every warp still gets a task (each
@@ -1907,7 +1962,8 @@ template <class T>
 __device__ __forceinline__ void tmul_staged(const TmulOp a, const TmulOp b, int nops, int v, int n, int kc, bool tri)
 {
     if constexpr (sizeof(T) == 8) {
-        if ((n & 1) == 0) tmul_staged_w<T, 2>(a, b, nops, v, n, kc, tri);
+        if (tmul_whole(n, kc)) cta_tmul_s(a, b, nops, v, n, kc);
+        else if ((n & 1) == 0) tmul_staged_w<T, 2>(a, b, nops, v, n, kc, tri);
         else tmul_staged_w<T, 1>(a, b, nops, v, n, kc, tri);
     } else {
         if ((n & 3) == 0) tmul_staged_w<T, 4>(a, b, nops, v, n, kc, tri);

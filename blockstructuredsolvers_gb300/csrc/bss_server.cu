@@ -26,14 +26,12 @@ namespace {
 
 // scratch of the builder (FP64, n x n unless noted)
 struct KfScratch {
-    double *QF, *FQF, *HRH, *RH /* m x n */, *Aint, *Afirst, *Alast, *Bup, *p0x /* n */;
-    static size_t doubles(long long n, long long m) { return 7 * n * n + m * n + n; }
+    double *QF, *RH /* m x n */, *Aint, *Afirst, *Alast, *Bup, *p0x /* n */;
+    static size_t doubles(long long n, long long m) { return 5 * n * n + m * n + n; }
     void carve(double *base, long long n, long long m)
     {
         QF = base;
-        FQF = QF + n * n;
-        HRH = FQF + n * n;
-        RH = HRH + n * n;
+        RH = QF + n * n;
         Aint = RH + m * n;
         Afirst = Aint + n * n;
         Alast = Afirst + n * n;

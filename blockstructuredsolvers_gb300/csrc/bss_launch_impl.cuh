@@ -304,19 +304,25 @@ static int sweep_threads(const SolveArgs<T> &a, bool staged)
 }
 
 // Whether a sweep starts under the one before it (see pdl_release_next), the
-// larger of the two levels having `partitions`.  It gains the launch and the
-// first loads, 2 to 3 us a level.  But CTAs that start early go where there is
-// room, two to an SM where two fit, and stay there; when the earlier level
-// fills the SMs that doubles a step's time.  Unstaged steps are long, and
-// several CTAs always fit.  Solve, all levels chained / by this rule / none,
-// separate launches in stream order with assembled right-hand sides = 1: FP64 N = 4000 n = 20 k = 16 1.41 / 0.81 /
-// 0.71, N = 964 n = 72 k = 1 1.14 / 1.01 / 1.01; N = 4000 n = 16 k = 1 0.52 / 0.48 /
-// 0.53, FP32 n = 40 k = 16 1.14 / 0.97 / 1.01, n = 16 k = 1 0.62 / 0.61 / 0.71,
-// N = 33 n = 32 k = 1 (few partitions) FP64 0.56 / 0.55 / 0.66, FP32 0.70 / 0.69 / 0.89.
-static bool chains(bool staged, size_t smem, long long partitions)
+// larger of the two levels having `blocks` in `partitions`.  It gains the
+// launch and the first loads, 2 to 3 us a level.  But CTAs that start early go
+// where there is room, two to an SM where two fit, and stay there; when the
+// earlier level fills the SMs that doubles a step's time.  Unstaged steps are
+// long, and several CTAs always fit.  Solve, all levels chained / chained by
+// this rule / in order, launches in order with assembled right-hand sides = 1:
+// FP64 N = 4000 n = 20 k = 16 1.41 / 0.81 / 0.71, N = 964 n = 72 k = 1 1.14 / 1.01 /
+// 1.01, N = 4000 n = 16 k = 1 0.52 / 0.48 / 0.53; FP32 N = 4000 n = 40 k = 16 1.14 /
+// 0.97 / 1.01, n = 16 k = 1 0.62 / 0.61 / 0.71; few partitions, N = 33 n = 32 k = 1
+// FP64 0.56 / 0.55 / 0.66, FP32 0.70 / 0.69 / 0.89.
+// A light step (FP32, or an FP64 product of 2048 FMAs and fewer) loses little
+// to a level that no more than fills the SMs, or to short partitions, and is
+// chained there too (N = 1000, n = 16, k = 16, FP32: 124 us, 130 in order).
+template <class T>
+static bool chains(const SolveArgs<T> &a, bool staged, size_t smem, long long blocks, long long partitions)
 {
-    const bool two_fit = 2 * smem <= 227 * 1024;
-    return staged && !(two_fit && 2 * partitions > device_sms());
+    if (!staged || 2 * smem > 227 * 1024) return staged;
+    const bool light = sizeof(T) == 4 || a.n * a.n * a.kc <= 2048;
+    return light ? partitions <= device_sms() || blocks < 4 * partitions : 2 * partitions <= device_sms();
 }
 
 template <class T>
@@ -344,7 +350,7 @@ cudaError_t launch_chain_fwd(const SolveArgs<T> &a, cudaStream_t s)
     cudaError_t e = set_solve_smem<T>((const void *)kern, smem);
     if (e != cudaSuccess) return e;
     const unsigned grid = a.seq ? 1u : (unsigned)a.Q;
-    if (a.chained && chains(staged, smem, a.fine_Q)) e = launch_chained(kern, grid, sweep_threads<T>(a, staged), smem, s, a);
+    if (a.chained && chains(a, staged, smem, a.fine_N, a.fine_Q)) e = launch_chained(kern, grid, sweep_threads<T>(a, staged), smem, s, a);
     else kern<<<grid, sweep_threads<T>(a, staged), smem, s>>>(a);
     count_launch();
     return e != cudaSuccess ? e : cudaGetLastError();
@@ -367,7 +373,7 @@ cudaError_t launch_chain_bwd(const SolveArgs<T> &a, cudaStream_t s)
     auto kern = staged ? chain_bwd_kernel<T, Tsep, true> : chain_bwd_kernel<T, Tsep, false>;
     cudaError_t e = set_solve_smem<T>((const void *)kern, smem);
     if (e != cudaSuccess) return e;
-    if (a.chained && chains(staged, smem, a.Q)) e = launch_chained(kern, (unsigned)a.Q, sweep_threads<T>(a, staged), smem, s, a);
+    if (a.chained && chains(a, staged, smem, a.N, a.Q)) e = launch_chained(kern, (unsigned)a.Q, sweep_threads<T>(a, staged), smem, s, a);
     else kern<<<(unsigned)a.Q, sweep_threads<T>(a, staged), smem, s>>>(a);
     count_launch();
     return e != cudaSuccess ? e : cudaGetLastError();

@@ -1929,7 +1929,7 @@ static __device__ __noinline__ void cta_tmul_s(const TmulOp a, const TmulOp b, i
 // filled, 1.02 / 0.86.)
 __device__ __forceinline__ bool tmul_whole(int n, int kc)
 {
-    if (kc < 12 || n % 2 != 0 || n > (int)blockDim.x) return false;
+    if (kc < 12 || n > (int)blockDim.x) return false;
     const int padded = ((n + 7) & ~7) * ((n + 7) & ~7);
     return n <= 4 || (padded > 2 * n * n && kc > 24) ||
            (n * kc > 3 * (int)blockDim.x && (kc + 3) / 4 * n <= (int)blockDim.x);
@@ -1954,6 +1954,12 @@ __device__ __forceinline__ void tmul_staged_w(const TmulOp a, const TmulOp b, in
             else if (tasks >= 2 * nw) cta_tmul_t<T, W, 4, 2>(a, b, nops, v, n, kc, tri);
             else cta_tmul_t<T, W, 4, 1>(a, b, nops, v, n, kc, tri);
         } else {
+            if constexpr (sizeof(T) == 8 && W == 2) {
+                if (tmul_whole(n, kc)) {
+                    cta_tmul_s(a, b, nops, v, n, kc);
+                    break;
+                }
+            }
             cta_tmul_t<T, W, 4, 1>(a, b, nops, v, n, kc, tri);
         }
     }
@@ -1962,8 +1968,7 @@ template <class T>
 __device__ __forceinline__ void tmul_staged(const TmulOp a, const TmulOp b, int nops, int v, int n, int kc, bool tri)
 {
     if constexpr (sizeof(T) == 8) {
-        if (tmul_whole(n, kc)) cta_tmul_s(a, b, nops, v, n, kc);
-        else if ((n & 1) == 0) tmul_staged_w<T, 2>(a, b, nops, v, n, kc, tri);
+        if ((n & 1) == 0) tmul_staged_w<T, 2>(a, b, nops, v, n, kc, tri);
         else tmul_staged_w<T, 1>(a, b, nops, v, n, kc, tri);
     } else {
         if ((n & 3) == 0) tmul_staged_w<T, 4>(a, b, nops, v, n, kc, tri);

@@ -25,11 +25,11 @@
 // of two h_k ~ sqrt(S_kk): 2^h_k V(k, .) and 2^-h_k Z(k, .), which cancel in the
 // product, are two operands of one scale (S balanced has diagonal [1, 4)); it
 // is an integer added to the exponents that the cut works with, and a result
-// does not depend on a D of powers of two at all.  D in 2^+-27, 19 blocks:
-// 2e-3 to 0.2 off without the balance, 1e-15 with it, at no cost (N = 16384,
-// n = 64: 10.10 -> 10.09 ms: S_LL and the cuts also moved between pivot tiles).  (An FMA chain also
-// keeps the small terms of a single balanced row; digits do not.)  Rows with an
-// infinity or NaN give NaN.
+// does not depend on a D of powers of two at all.  D in 2^+-40, 19 blocks: 0.2
+// off without the balance, within 1e-12 with it, in the same time (N = 16384,
+// n = 64: 10.1 ms; the step's asides are spread better as well).  What an FMA
+// chain keeps and digits do not: terms of one balanced row that are smaller
+// than 2^-54 of its largest.  Rows with an infinity or NaN give NaN.
 //
 // A step of the chain (NB = 64 or 32, the block padded with the identity):
 //   P1 = [W_{i-1} | Y_{i-1}]^T W_{i-1}   -> S = A_i - W^T W (slot 0 rows), Z_i^T = -Y^T W (slot 1 rows)
@@ -54,7 +54,7 @@
 // 1.4K for NB = 32, against 131K and 16K for one product on the FP64 pipe):
 // plain FP64 factor + solve of N = 16384, n = 64: 35.6 -> 11.3 ms; N = 1531,
 // n = 37, k = 3: 6.42 -> 2.68 ms; N = 100, n = 32: 679 -> 435 us (10.1 ms, 2.1 ms
-// and 378 us with the sweeps as they are now).  A 64-wide step takes ~145K cycles:
+// and 372 us with the sweeps as they are now).  A 64-wide step takes ~145K cycles:
 // 49K in the four pivot tiles, 46K in the Cholesky's other FP64 products, 31K
 // cutting and putting together digits, 15K in MMAs.
 #pragma once
